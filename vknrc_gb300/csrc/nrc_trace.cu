@@ -12,17 +12,34 @@
 
 #include <cmath>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "nrc_common.cuh"
 #include "nrc_kernels.h"
 
+// A four-wide node: for each axis the low and the high planes of its four slots,
+// so that a ray loads its near and far planes as two 16-byte words chosen by the
+// sign of its direction. 128 bytes, one cache line.
+struct __align__(128) WideNode {
+  float4 plane[6];  // low x, high x, low y, high y, low z, high z; an empty slot's low planes above its high ones
+  uint32_t node0;   // first child node
+  uint32_t tri0;    // first triangle (in the leaf array)
+  // bit 24 + s: slot s holds a node; bits 3s .. 3s+2: the triangles (at most
+  // three) of slot s. Nodes and triangles are stored in the order of those bits.
+  uint32_t contents;
+  uint32_t unused[5];
+};
+static_assert(sizeof(WideNode) == 128, "one cache line");
+
 struct nrc_bvh {
   int device = 0;
   uint32_t tris = 0, nodes = 0;
-  void* block = nullptr;  // triangles, then nodes
-  const float4* tri = nullptr;  // 3 x float4 per triangle: v0.xyz prim, v1.xyz inst, v2.xyz pad
-  const uint4* node = nullptr;  // 2 x uint4 per node: lo.xyz left, hi.xyz right
+  void* block = nullptr;          // the four arrays below
+  const float4* tri = nullptr;    // 3 x float4 per triangle: v0.xyz prim, v1.xyz inst, v2.xyz pad
+  const float4* guard = nullptr;  // 2 x float4 per triangle: lo.xyz, hi.xyz of its guard box
+  const float4* leaf = nullptr;   // 3 x float4 per triangle in tree order: v0.xyz triangle, (v1 - v0).xyz, (v2 - v0).xyz
+  const WideNode* wide = nullptr;
 };
 
 namespace nrc {
@@ -350,15 +367,22 @@ __device__ Hit make_hit(const nrc_scene& S, const float* lut, uint32_t prim, uin
 // ------------------------------------------------------------- bvh trace --
 struct TriView {
   const float4* tri;
-  const uint4* node;
+  const float4* guard;
+  const float4* leaf;
+  const WideNode* wide;
   uint32_t tris;
 };
 
+// The binary tree under the wide one is at most kMaxHeight + 31 high, and a
+// traversal stacks at most one entry per level.
+constexpr uint32_t kMaxHeight = 48;
+constexpr int kStack = kMaxHeight + 32;
+
 // Moller-Trumbore: t and barycentrics (u: vertex 1, v: vertex 2) when the ray
 // meets the triangle with t in [tmin, tmax].
-__device__ bool intersect(const float4* T, Ray r, float tmin, float tmax, float& t, float& u, float& v) {
-  const float4 a = T[0], b = T[1], c = T[2];
-  const V3 v0 = v3(a.x, a.y, a.z), e1 = sub(v3(b.x, b.y, b.z), v0), e2 = sub(v3(c.x, c.y, c.z), v0);
+__device__ __forceinline__ bool intersect(float4 a, float4 b, float4 c, Ray r, float tmin, float tmax, float& t, float& u,
+                                          float& v) {
+  const V3 v0 = v3(a.x, a.y, a.z), e1 = v3(b.x, b.y, b.z), e2 = v3(c.x, c.y, c.z);
   const V3 p = cross(r.d, e2);
   const float det = dot(e1, p);
   if (det == 0.0f || det != det) return false;
@@ -373,47 +397,145 @@ __device__ bool intersect(const float4* T, Ray r, float tmin, float tmax, float&
   return t >= tmin && t <= tmax;
 }
 
+// Slab test of a triangle's guard box (its parent's padded box in the binary
+// radix tree). A grazing ray's triangle test can accept a point well off the
+// triangle; a hit counts only if the ray also meets this box, so the hits do
+// not depend on how the wide tree groups and quantises its boxes (which all
+// contain the guard boxes).
+__device__ __forceinline__ bool guard_hit(float4 lo, float4 hi, V3 o, float ix, float iy, float iz, float tmin, float bt) {
+  const float x0 = (lo.x - o.x) * ix, x1 = (hi.x - o.x) * ix;
+  const float y0 = (lo.y - o.y) * iy, y1 = (hi.y - o.y) * iy;
+  const float z0 = (lo.z - o.z) * iz, z1 = (hi.z - o.z) * iz;
+  const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
+  const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), bt));
+  return tn <= tf * 1.00001f + 1e-7f;
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // Closest triangle along the ray in [tmin, tmax]; equal distances go to the lower
-// triangle index. Returns the triangle index or -1. Kept out of line: the
-// kernel traces from several call sites, and one shared copy of the traversal
-// loop keeps the kernel's hot code within the instruction cache (measured 17%
-// faster at 1080p than inlining it everywhere).
-__device__ __noinline__ int trace_closest(const TriView& B, Ray r, float tmin, float tmax, float& bt, float& bu,
+// triangle index. Returns the triangle index or -1. Kept out of line, which
+// keeps its registers apart from the shading's (inlined: 1.73 against
+// 1.68 ms).
+// The lanes that call together step together: each iteration is one node for
+// every lane with a node to visit, or one triangle test for every lane with
+// triangles pending, chosen so that steps run with many lanes (left to diverge
+// freely, the loops ran with 6 lanes per instruction). A lane goes on visiting
+// nodes until the triangles of two nodes are pending.
+__device__ __noinline__ int trace_closest(const TriView& B, Ray r, float tmin, float tmax, float& bt_out, float& bu,
                                           float& bv) {
   if (B.tris == 0) return -1;
   const float ix = fabsf(r.d.x) > 1e-20f ? 1.0f / r.d.x : copysignf(1e20f, r.d.x);
   const float iy = fabsf(r.d.y) > 1e-20f ? 1.0f / r.d.y : copysignf(1e20f, r.d.y);
   const float iz = fabsf(r.d.z) > 1e-20f ? 1.0f / r.d.z : copysignf(1e20f, r.d.z);
+  const float ox = -r.o.x * ix, oy = -r.o.y * iy, oz = -r.o.z * iz;  // coordinate p is met at p * i + o
+  const int sx = ix >= 0.0f ? 0 : 1, sy = iy >= 0.0f ? 0 : 1, sz = iz >= 0.0f ? 0 : 1;  // which of the planes is near
+  // A ray with a NaN meets nothing (every comparison of the triangle test fails).
+  const float sum = (r.o.x + r.o.y + r.o.z) + (r.d.x + r.d.y + r.d.z);
+  constexpr uint32_t kRoot = (1u << 24) | 1u;
   int best = -1;
-  bt = tmax;
-  uint32_t stack[64];
+  float bt = tmax;
+  // A group of sibling nodes: the first one, and a word with the slots still to
+  // visit (bits 24..27), the nearest of them when the group was met (bits 8, 9)
+  // and the slots holding nodes (bits 0..3). The root is slot 0 of its own group.
+  uint2 stack[kStack];
   int sp = 0;
-  stack[sp++] = B.tris == 1 ? kLeaf : 0u;
-  while (sp > 0) {
-    const uint32_t id = stack[--sp];
-    if (id & kLeaf) {
-      const uint32_t ti = id & ~kLeaf;
-      float t, u, v;
-      if (intersect(B.tri + size_t(ti) * 3, r, tmin, bt, t, u, v) &&
-          (t < bt || (t == bt && (best < 0 || static_cast<int>(ti) < best)))) {
-        best = static_cast<int>(ti);
-        bt = t;
-        bu = u;
-        bv = v;
+  uint32_t base = 0, group = sum == sum ? kRoot : 0u;
+  uint32_t tri0 = 0, tset = 0, tri1 = 0, tset1 = 0;  // pending triangles of two nodes: first, present << 12 | hit
+  bool strict = false;  // test the guard box of every hit, not only of the closest
+  const uint32_t lanes = __activemask();
+  while (true) {
+    const bool has_tri = tset != 0u, has_node = group >= (1u << 24) && tset1 == 0u;
+    const uint32_t want_tri = __ballot_sync(lanes, has_tri), want_node = __ballot_sync(lanes, has_node);
+    if ((want_tri | want_node) == 0u) {
+      // the closest hit counts if it meets its guard box; if not (a grazing
+      // ray, rarely), the lane starts again, testing every hit's
+      const bool again = best >= 0 && !strict &&
+                         !guard_hit(__ldg(B.guard + size_t(best) * 2), __ldg(B.guard + size_t(best) * 2 + 1), r.o, ix, iy,
+                                    iz, tmin, tmax);
+      if (__ballot_sync(lanes, again) == 0u) break;
+      if (again) {
+        strict = true;
+        best = -1;
+        bt = tmax;
+        base = 0u;
+        group = kRoot;
       }
       continue;
     }
-    const uint4 lo = B.node[size_t(id) * 2], hi = B.node[size_t(id) * 2 + 1];
-    const float x0 = (__uint_as_float(lo.x) - r.o.x) * ix, x1 = (__uint_as_float(hi.x) - r.o.x) * ix;
-    const float y0 = (__uint_as_float(lo.y) - r.o.y) * iy, y1 = (__uint_as_float(hi.y) - r.o.y) * iy;
-    const float z0 = (__uint_as_float(lo.z) - r.o.z) * iz, z1 = (__uint_as_float(hi.z) - r.o.z) * iz;
-    const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-    const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), bt));
-    if (!(tn <= tf * 1.00001f + 1e-7f)) continue;  // conservative: the boxes are padded too
-    if (sp + 2 > 64) continue;  // cannot happen for a radix tree of < 2^30 leaves (depth <= 63)
-    stack[sp++] = lo.w;
-    stack[sp++] = hi.w;
+    if (want_node == 0u || 3 * __popc(want_tri) >= 2 * __popc(want_tri | want_node)) {
+      if (has_tri) {
+        const uint32_t bit = tset & (0u - tset);
+        const float4* T = B.leaf + size_t(tri0 + __popc((tset >> 12) & (bit - 1u))) * 3;
+        const float4 a = __ldg(T), b = __ldg(T + 1), c = __ldg(T + 2);
+        tset ^= bit;
+        if ((tset & 0xFFFu) == 0u) {
+          tri0 = tri1;
+          tset = tset1;
+          tset1 = 0u;
+        }
+        const int ti = __float_as_int(a.w);
+        float t, u, v;
+        if (intersect(a, b, c, r, tmin, bt, t, u, v) && (t < bt || best < 0 || ti < best) &&
+            (!strict || guard_hit(__ldg(B.guard + size_t(ti) * 2), __ldg(B.guard + size_t(ti) * 2 + 1), r.o, ix, iy, iz, tmin,
+                                  tmax))) {
+          best = ti;
+          bt = t;
+          bu = u;
+          bv = v;
+        }
+      }
+    } else if (has_node) {
+      uint32_t bit = group & (1u << (24u + ((group >> 8) & 3u)));
+      const uint32_t left = group & 0x0F000000u;
+      bit = bit != 0u ? bit : left & (0u - left);
+      group ^= bit;
+      const WideNode* N = B.wide + (base + __popc(group & ((bit >> 24) - 1u)));
+      const float4 nx = __ldg(N->plane + sx), fx = __ldg(N->plane + (1 - sx)), ny = __ldg(N->plane + 2 + sy),
+                   fy = __ldg(N->plane + (3 - sy)), nz = __ldg(N->plane + 4 + sz), fz = __ldg(N->plane + (5 - sz));
+      const uint4 m = __ldg(reinterpret_cast<const uint4*>(&N->node0));
+      uint32_t hit = 0, near = 0xFFFFFFFFu;
+      auto slot = [&](float x0, float y0, float z0, float x1, float y1, float z1, uint32_t s) {
+        const float tn = fmaxf(max3(fmaf(x0, ix, ox), fmaf(y0, iy, oy), fmaf(z0, iz, oz)), tmin);
+        const float tf = fminf(min3(fmaf(x1, ix, ox), fmaf(y1, iy, oy), fmaf(z1, iz, oz)), bt);
+        const bool in = tn <= fmaf(tf, 1.0001f, 1e-6f);
+        hit |= in ? (7u << (3 * s)) | (1u << (24 + s)) : 0u;
+        near = min(near, in ? (__float_as_uint(tn) & ~3u) | s : 0xFFFFFFFFu);  // tn >= 0: its bits are ordered
+      };
+      slot(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, 0);
+      slot(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, 1);
+      slot(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, 2);
+      slot(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, 3);
+      hit &= m.z;
+      const uint32_t set = (hit & 0xFFFu) != 0u ? ((m.z & 0xFFFu) << 12) | (hit & 0xFFFu) : 0u;
+      const bool first = tset == 0u;
+      tri1 = first ? tri1 : m.y;
+      tset1 = first ? 0u : set;
+      tri0 = first ? m.y : tri0;
+      tset = first ? set : tset;
+      // down into the children met; else on to the siblings left, else to the last group stacked
+      const uint32_t below = (hit & 0x0F000000u) | (m.z >> 24) | ((near & 3u) << 8);
+      const bool down = below >= (1u << 24), rest = group >= (1u << 24);
+      if (down && rest) stack[sp++] = make_uint2(base, group);
+      if (!down && !rest && sp > 0) {
+        const uint2 e = stack[--sp];
+        base = e.x;
+        group = e.y;
+      }
+      base = down ? m.x : base;
+      group = down ? below : group;
+    }
   }
+  bt_out = bt;
   return best;
 }
 
@@ -485,109 +607,92 @@ __device__ __forceinline__ uint32_t dst_train(uint32_t b, uint32_t l, uint32_t r
   return ((b | (l << 2) | (r << 16)) << 1) | 1u;
 }
 
-// The secondary hit of a traced ray (GetRayQueryHit) or false for a miss.
-__device__ bool trace_hit(const TraceArgs& A, Ray ray, Hit& h) {
-  float t, u, v;
-  const int ti = trace_closest(A.bvh, ray, kTMin, kTMax, t, u, v);
-  if (ti < 0) return false;
-  const float4* T = A.bvh.tri + size_t(ti) * 3;
-  const nrc_scene& S = A.sc.s;
-  const uint32_t prim = __float_as_uint(T[0].w), inst = __float_as_uint(T[1].w);
-  const V3 v0 = scene_vertex(S, inst, prim, 0), v1 = scene_vertex(S, inst, prim, 1), v2 = scene_vertex(S, inst, prim, 2);
-  h = make_hit(S, A.sc.lut, prim, inst, u, v, v0, v1, v2, cross(sub(v1, v0), sub(v2, v0)), ray);
-  return true;
-}
-
 struct Result {
   V3 bias, factor;
 };
 
-// PathTrace, path_tracer.comp:208-250 (the method is warp-uniform here).
-__device__ Result path_trace(const TraceArgs& A, Hit hit, Ray ray, uint32_t method, Rng& rng, uint32_t x, uint32_t y) {
+// The path of one pixel from its camera ray: PathTrace (path_tracer.comp:208-250)
+// or, for training pixels, ExtendedPathTrace (:252-375), which follows the path
+// past the point where the screen's part of it ends (`suffix`) and writes train
+// records. Both walk the same loop, so the kernel holds one copy of the hit
+// record and the BRDF step: with a copy per call site its hot code did not fit
+// the instruction cache. The method and `train` are warp-uniform.
+__device__ __forceinline__ Result trace_path(const TraceArgs& A, const float* lut, Ray ray, uint32_t method, bool train, Rng& rng,
+                             uint32_t x, uint32_t y) {
+  V3 lights[kMaxBounce], colors[kMaxBounce];  // training: of the vertex after vertex i
+  nrc_packed_input inputs[kMaxBounce];
   V3 radiance = v3(0.f, 0.f, 0.f), acc = v3(1.f, 1.f, 1.f);
-  Step info = brdf_step(hit, ray, rng);
-  radiance = add(radiance, mul(acc, hit.emission));
-  acc = mul(acc, info.color);
-  ray = info.ray;
-  const float c_a0 =
-      method == NRC_METHOD_NONE ? __int_as_float(0x7F800000) : kC * info.dist2 / (4.0f * kPi * info.cosine);
-  float sqrt_a_sum = 0.0f;
-  if (method != NRC_METHOD_CACHE) {
-    for (int bounce = 1; bounce < kMaxBounce && sqrt_a_sum * sqrt_a_sum <= c_a0; ++bounce) {
-      if (trace_hit(A, ray, hit)) {
-        info = brdf_step(hit, ray, rng);
+  Result result;
+  const nrc_scene& S = A.sc.s;
+  float c_a0 = 0.0f, sqrt_a_sum = 0.0f;
+  bool suffix = false, light_terminate = false;
+  int bounce = 0;  // vertices so far
+  Hit hit;
+  while (true) {
+    float t, u, v;
+    const int ti = trace_closest(A.bvh, ray, bounce == 0 ? 0.0f : kTMin, bounce == 0 ? __int_as_float(0x7F800000) : kTMax,
+                                 t, u, v);
+    if (ti < 0) {
+      if (bounce == 0) return Result{v3(kConstLight, kConstLight, kConstLight), v3(0.f, 0.f, 0.f)};
+      if (!suffix) radiance = add(radiance, scale(acc, kConstLight));
+      if (!train) return Result{radiance, acc};
+      lights[bounce - 1] = v3(kConstLight, kConstLight, kConstLight);
+      light_terminate = true;
+    } else {
+      const float4* T = A.bvh.tri + size_t(ti) * 3;
+      const uint32_t prim = __float_as_uint(T[0].w), inst = __float_as_uint(T[1].w);
+      const V3 v0 = scene_vertex(S, inst, prim, 0), v1 = scene_vertex(S, inst, prim, 1),
+               v2 = scene_vertex(S, inst, prim, 2);
+      const V3 v01 = sub(v1, v0), v02 = sub(v2, v0), n = cross(v01, v02);
+      if (bounce == 0) {  // GetVBufferHit's barycentrics: the ray against the triangle's plane
+        const V3 q = cross(sub(ray.o, v0), ray.d);
+        const float d = 1.0f / dot(ray.d, n);
+        u = d * dot(neg(q), v02);
+        v = d * dot(q, v01);
+      }
+      hit = make_hit(S, lut, prim, inst, u, v, v0, v1, v2, n, ray);
+      const Step info = brdf_step(hit, ray, rng);
+      if (!suffix) {
         radiance = add(radiance, mul(acc, hit.emission));
         acc = mul(acc, info.color);
-        ray = info.ray;
-        sqrt_a_sum = sqrt_a_sum + sqrtf(info.dist2 / (info.pdf * info.cosine));
-      } else {
-        radiance = add(radiance, scale(acc, kConstLight));
-        return Result{radiance, acc};
       }
-    }
-  }
-  if (method != NRC_METHOD_NONE) push_eval(A, dst_screen(x, y), make_input(hit, ray.d));
-  return Result{radiance, acc};
-}
-
-// ExtendedPathTrace, path_tracer.comp:252-375.
-__device__ Result extended_trace(const TraceArgs& A, Hit hit, Ray ray, uint32_t method, Rng& rng, uint32_t x,
-                                 uint32_t y) {
-  V3 lights[kMaxBounce], colors[kMaxBounce];
-  nrc_packed_input inputs[kMaxBounce];
-  for (int i = 0; i < kMaxBounce; ++i) {
-    colors[i] = v3(1.f, 1.f, 1.f);
-    lights[i] = v3(0.f, 0.f, 0.f);
-  }
-  V3 acc = v3(1.f, 1.f, 1.f), radiance = v3(0.f, 0.f, 0.f);
-  bool light_terminate = false;
-  Step info = brdf_step(hit, ray, rng);
-  radiance = add(radiance, mul(acc, hit.emission));
-  acc = mul(acc, info.color);
-  ray = info.ray;
-  Result result{radiance, acc};
-  inputs[0] = make_input(hit, ray.d);
-  const float c_a0 = kC * info.dist2 / (4.0f * kPi * info.cosine);
-  float sqrt_a_sum = 0.0f;
-  int bounce = 1;
-  for (; bounce < kMaxBounce && sqrt_a_sum * sqrt_a_sum <= c_a0; ++bounce) {
-    if (trace_hit(A, ray, hit)) {
-      info = brdf_step(hit, ray, rng);
-      radiance = add(radiance, mul(acc, hit.emission));
-      acc = mul(acc, info.color);
       ray = info.ray;
-      sqrt_a_sum = sqrt_a_sum + sqrtf(info.dist2 / (info.pdf * info.cosine));
-      lights[bounce - 1] = hit.emission;
-      colors[bounce - 1] = info.color;
-      inputs[bounce] = make_input(hit, ray.d);
-    } else {
-      radiance = add(radiance, scale(acc, kConstLight));
-      lights[bounce - 1] = v3(kConstLight, kConstLight, kConstLight);
-      light_terminate = true;
-      break;
+      if (bounce == 0)
+        c_a0 = method == NRC_METHOD_NONE ? __int_as_float(0x7F800000) : kC * info.dist2 / (4.0f * kPi * info.cosine);
+      else
+        sqrt_a_sum = sqrt_a_sum + sqrtf(info.dist2 / (info.pdf * info.cosine));
+      if (train) {
+        inputs[bounce] = make_input(hit, ray.d);
+        lights[bounce] = v3(0.f, 0.f, 0.f);
+        colors[bounce] = v3(1.f, 1.f, 1.f);
+        if (bounce > 0) {
+          lights[bounce - 1] = hit.emission;
+          colors[bounce - 1] = info.color;
+        }
+      }
+      if (bounce == 0) result = Result{radiance, acc};
+      ++bounce;
     }
-  }
-  if (method == NRC_METHOD_CACHE) {
-    push_eval(A, dst_screen(x, y), inputs[0]);
-  } else {
-    result = Result{radiance, acc};
-    if (!light_terminate) push_eval(A, dst_screen(x, y), inputs[bounce - 1]);
-  }
-  sqrt_a_sum = 0.0f;
-  light_terminate = false;
-  for (; bounce < kMaxBounce && sqrt_a_sum * sqrt_a_sum <= c_a0; ++bounce) {
-    if (trace_hit(A, ray, hit)) {
-      info = brdf_step(hit, ray, rng);
-      ray = info.ray;
-      sqrt_a_sum = sqrt_a_sum + sqrtf(info.dist2 / (info.pdf * info.cosine));
-      lights[bounce - 1] = hit.emission;
-      colors[bounce - 1] = info.color;
-      inputs[bounce] = make_input(hit, ray.d);
-    } else {
-      lights[bounce - 1] = v3(kConstLight, kConstLight, kConstLight);
-      light_terminate = true;
-      break;
+    // does the path go on? (a cache query ends the screen's part at the first vertex)
+    const bool grow = !light_terminate && bounce < kMaxBounce && sqrt_a_sum * sqrt_a_sum <= c_a0;
+    if (!train) {
+      if (grow && method != NRC_METHOD_CACHE) continue;
+      if (method != NRC_METHOD_NONE) push_eval(A, dst_screen(x, y), make_input(hit, ray.d));
+      return Result{radiance, acc};
     }
+    if (grow) continue;
+    if (!suffix) {  // the screen's record; then the training suffix, its spread measured anew
+      if (method == NRC_METHOD_CACHE) {
+        push_eval(A, dst_screen(x, y), inputs[0]);
+      } else {
+        result = Result{radiance, acc};
+        if (!light_terminate) push_eval(A, dst_screen(x, y), inputs[bounce - 1]);
+      }
+      suffix = true;
+      sqrt_a_sum = 0.0f;
+      if (!light_terminate && bounce < kMaxBounce && 0.0f <= c_a0) continue;
+    }
+    break;
   }
   // clamp(uint(u * 4), 0, 3) with u in [0, 1]
   uint32_t batch = static_cast<uint32_t>(rng.next() * static_cast<float>(NRC_TRAIN_BATCH_COUNT));
@@ -621,10 +726,10 @@ __device__ Result extended_trace(const TraceArgs& A, Hit hit, Ray ray, uint32_t 
 
 // main(), path_tracer.comp:377-420: 8 x 8 threads per block, warps of 32
 // consecutive threads (4 rows), the warp standing in for the subgroup.
-// 16 blocks of 64 threads per SM (64 registers): more warps to hide the BVH
-// loads measured faster than fewer, spill-free warps (2.67 against 3.03 ms at
-// 1080p with 12 blocks). A near-child-first traversal (both children's boxes
-// tested at each node) measured slower here (2.79 ms).
+// 16 blocks of 64 threads per SM (64 registers): 12 blocks without spills and
+// with the traversal inlined measured slower (1.85 against 1.68 ms for 8-bounce
+// paths at 960 x 540, 1.83 against 1.74 ms for cache paths at 1920 x 1080; 2.72 ms
+// over the binary tree).
 __global__ void __launch_bounds__(64, 16) path_trace_kernel(const __grid_constant__ TraceArgs A) {
   extern __shared__ float lut_s[];
   for (int i = threadIdx.y * 8 + threadIdx.x; i < 256; i += 64) lut_s[i] = A.sc.lut[i];
@@ -643,31 +748,13 @@ __global__ void __launch_bounds__(64, 16) path_trace_kernel(const __grid_constan
     if (lane == first) train = rng.next() < A.p.train_probability;
     train = __shfl_sync(active, train ? 1 : 0, first) != 0;
   }
-  // primary hit (the V-buffer's primitive and instance), then GetVBufferHit
+  // the camera ray (the primary hit replaces the V-buffer's primitive and instance)
   const float cx = (static_cast<float>(x) + 0.5f) / static_cast<float>(A.p.width) * 2.0f - 1.0f;
   const float cy = (static_cast<float>(y) + 0.5f) / static_cast<float>(A.p.height) * 2.0f - 1.0f;
   const V3 look = v3(A.p.look[0], A.p.look[1], A.p.look[2]), side = v3(A.p.side[0], A.p.side[1], A.p.side[2]),
            up = v3(A.p.up[0], A.p.up[1], A.p.up[2]);
   Ray ray{v3(A.p.origin[0], A.p.origin[1], A.p.origin[2]), normalize(add(add(look, scale(side, cx)), scale(up, cy)))};
-  Result res;
-  float pt, pu, pv;
-  const int ti = trace_closest(A.bvh, ray, 0.0f, __int_as_float(0x7F800000), pt, pu, pv);
-  if (ti < 0) {
-    res = Result{v3(kConstLight, kConstLight, kConstLight), v3(0.f, 0.f, 0.f)};
-  } else {
-    const float4* T = A.bvh.tri + size_t(ti) * 3;
-    const nrc_scene& S = A.sc.s;
-    const uint32_t prim = __float_as_uint(T[0].w), inst = __float_as_uint(T[1].w);
-    const V3 v0 = scene_vertex(S, inst, prim, 0), v1 = scene_vertex(S, inst, prim, 1),
-             v2 = scene_vertex(S, inst, prim, 2);
-    // GetVBufferHit's barycentrics: the ray against the triangle's plane
-    const V3 v01 = sub(v1, v0), v02 = sub(v2, v0), v0o = sub(ray.o, v0);
-    const V3 n = cross(v01, v02), q = cross(v0o, ray.d);
-    const float d = 1.0f / dot(ray.d, n);
-    const float u = d * dot(neg(q), v02), v = d * dot(q, v01);
-    const Hit hit = make_hit(S, lut_s, prim, inst, u, v, v0, v1, v2, n, ray);
-    res = train ? extended_trace(A, hit, ray, method, rng, x, y) : path_trace(A, hit, ray, method, rng, x, y);
-  }
+  Result res = trace_path(A, lut_s, ray, method, train, rng, x, y);
   res.bias = normalize_rgb(res.bias);
   res.factor = normalize_rgb(res.factor);
   const size_t px = size_t(y) * A.p.width + x;
@@ -838,6 +925,270 @@ __global__ void refit_kernel(const float4* tri, int n, uint4* node, const uint32
   }
 }
 
+// The guard box of each triangle: its parent's padded box (unbounded for a lone
+// triangle). The clustering below starts from these boxes.
+__global__ void guard_kernel(int n, const uint4* node, const uint32_t* parent, float4* guard) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const float inf = __int_as_float(0x7F800000);
+  float4 lo = make_float4(-inf, -inf, -inf, 0.0f), hi = make_float4(inf, inf, inf, 0.0f);
+  if (n > 1) {
+    const uint32_t p = parent[(n - 1) + t];
+    const uint4 a = node[size_t(p) * 2], b = node[size_t(p) * 2 + 1];
+    lo = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.0f);
+    hi = make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), 0.0f);
+  }
+  guard[size_t(t) * 2] = lo;
+  guard[size_t(t) * 2 + 1] = hi;
+}
+
+// Parallel locally-ordered clustering (Meister and Bittner 2018) over the
+// triangles in Morton order: each cluster looks kSearch places to either side for
+// the one whose union with it has the least area; pairs that choose each other
+// merge; the survivors keep their order. Unlike the radix tree, a triangle much
+// larger than its neighbours (a wall beside a tessellated floor) joins late,
+// near the root, instead of stretching the boxes of everything above a small one.
+// Ids: a triangle in Morton order at [0, n), merged clusters from n on.
+constexpr int kSearch = 16, kClusterThreads = 256;
+constexpr uint32_t kLeafTris = 3;
+
+struct Clusters {
+  float4 *lo, *hi;  // box per id; lo.w triangles below, hi.w height (as bits)
+  uint2* child;     // of id n + i
+  uint32_t* nn;     // chosen neighbour (place) of each place
+  uint32_t* kept;   // survivors per block
+  uint32_t* counters;  // see kNextId ..
+  uint32_t n;
+};
+// Counters: the next cluster id; the clusters before and after a pass (in turn);
+// wide nodes and leaf triangles so far; the wide nodes up to each level (from 0).
+constexpr int kNextId = 0, kCount = 1, kWide = 3, kLeafs = 4, kLevelEnd = 5, kCounters = kLevelEnd + kStack + 3;
+
+__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
+  const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
+  return x * y + y * z + z * x;
+}
+
+// A triangle's box: the part of its guard box within a margin of the triangle
+// that is wide against what rounding can add to the triangle test's edges (a
+// triangle beside a wall has a guard box as large as the wall). Boxes are kept
+// within +-1e15, so that no term of the traversal's slab test overflows.
+__global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const float4* guard, const float4* tri,
+                                    uint32_t* ids) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= C.n) return;
+  const uint32_t t = order[i];
+  const float4 a = guard[size_t(t) * 2], b = guard[size_t(t) * 2 + 1];
+  float lo[3] = {a.x, a.y, a.z}, hi[3] = {b.x, b.y, b.z};
+  const float4 v0 = tri[size_t(t) * 3], v1 = tri[size_t(t) * 3 + 1], v2 = tri[size_t(t) * 3 + 2];
+  float tl[3] = {fminf(fminf(v0.x, v1.x), v2.x), fminf(fminf(v0.y, v1.y), v2.y), fminf(fminf(v0.z, v1.z), v2.z)};
+  float th[3] = {fmaxf(fmaxf(v0.x, v1.x), v2.x), fmaxf(fmaxf(v0.y, v1.y), v2.y), fmaxf(fmaxf(v0.z, v1.z), v2.z)};
+  float margin = 0.0f;
+  for (int k = 0; k < 3; ++k)
+    margin = fmaxf(margin, (th[k] - tl[k]) * 0.015625f + (fabsf(tl[k]) + fabsf(th[k])) * 1e-4f + 1e-6f);
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = fmaxf(lo[k], tl[k] - margin);
+    hi[k] = fminf(hi[k], th[k] + margin);
+  }
+  for (int k = 0; k < 3; ++k) {
+    if (!(lo[k] <= hi[k])) lo[k] = hi[k] = 0.0f;  // no finite vertex: the triangle is never hit
+    lo[k] = fminf(fmaxf(lo[k], -1e15f), 1e15f);
+    hi[k] = fminf(fmaxf(hi[k], -1e15f), 1e15f);
+  }
+  C.lo[i] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(1u));
+  C.hi[i] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(0u));
+  ids[i] = i;
+}
+
+// Equal areas choose the nearer place, then the pair that starts at an even
+// place, so that runs of equal boxes pair up. Clusters kMaxHeight high count as
+// infinitely far: what is left then pairs by place, which bounds the tree's height.
+// The passes run in batches, grids sized by the count before the batch: the
+// count of a pass is in counters[kCount + turn].
+__global__ void __launch_bounds__(kClusterThreads) nearest_kernel(Clusters C, const uint32_t* ids, int turn) {
+  const uint32_t count = C.counters[kCount + turn];
+  if (blockIdx.x * kClusterThreads >= count) return;
+  __shared__ float4 slo[kClusterThreads + 2 * kSearch], shi[kClusterThreads + 2 * kSearch];
+  const int base = static_cast<int>(blockIdx.x) * kClusterThreads - kSearch;
+  for (int k = threadIdx.x; k < kClusterThreads + 2 * kSearch; k += kClusterThreads) {
+    const int j = base + k;
+    if (j >= 0 && j < static_cast<int>(count)) {
+      slo[k] = C.lo[ids[j]];
+      shi[k] = C.hi[ids[j]];
+    }
+  }
+  __syncthreads();
+  const int i = base + kSearch + static_cast<int>(threadIdx.x);
+  if (i >= static_cast<int>(count)) return;
+  const float4 lo = slo[threadIdx.x + kSearch], hi = shi[threadIdx.x + kSearch];
+  float best_d = 0.0f;
+  uint32_t best_k = 0, best_j = 0xFFFFFFFFu;
+  for (int o = -kSearch; o <= kSearch; ++o) {
+    const int j = i + o;
+    if (o == 0 || j < 0 || j >= static_cast<int>(count)) continue;
+    const float4 a = slo[threadIdx.x + kSearch + o], b = shi[threadIdx.x + kSearch + o];
+    float d = half_area(make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), 0.0f),
+                        make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), 0.0f));
+    if (max(__float_as_uint(hi.w), __float_as_uint(b.w)) >= kMaxHeight) d = __int_as_float(0x7F800000);
+    const uint32_t key = 2u * static_cast<uint32_t>(abs(o)) + (static_cast<uint32_t>(min(i, j)) & 1u);
+    if (best_j == 0xFFFFFFFFu || d < best_d || (d == best_d && key < best_k)) {
+      best_d = d;
+      best_k = key;
+      best_j = static_cast<uint32_t>(j);
+    }
+  }
+  C.nn[i] = best_j;
+}
+
+// Place i survives unless it merges into a lower place.
+__device__ __forceinline__ bool survives(const Clusters& C, uint32_t i, uint32_t count) {
+  if (i >= count) return false;
+  const uint32_t j = C.nn[i];  // none (above i) for a lone cluster
+  return !(j < i && C.nn[j] == i);
+}
+
+__global__ void __launch_bounds__(kClusterThreads) kept_kernel(Clusters C, int turn) {
+  const uint32_t count = C.counters[kCount + turn];
+  if (blockIdx.x * kClusterThreads >= count) return;
+  const uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x;
+  const int k = __syncthreads_count(survives(C, i, count) ? 1 : 0);
+  if (threadIdx.x == 0) C.kept[blockIdx.x] = static_cast<uint32_t>(k);
+}
+
+__global__ void __launch_bounds__(kClusterThreads) merge_kernel(Clusters C, const uint32_t* ids, uint32_t* out,
+                                                                int turn) {
+  const uint32_t count = C.counters[kCount + turn];
+  if (blockIdx.x * kClusterThreads >= count) return;
+  __shared__ uint32_t before[kClusterThreads / 32], warps[kClusterThreads / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  // survivors of the blocks before this one
+  uint32_t sum = 0;
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kClusterThreads) sum += C.kept[b];
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  const uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x;
+  const bool keep = survives(C, i, count);
+  const uint32_t m = __ballot_sync(0xffffffffu, keep);
+  if (lane == 0) {
+    before[warp] = sum;
+    warps[warp] = __popc(m);
+  }
+  __syncthreads();
+  uint32_t at = __popc(m & ((1u << lane) - 1u));
+  for (uint32_t w = 0; w < kClusterThreads / 32; ++w) {
+    at += before[w];
+    if (w < warp) at += warps[w];
+  }
+  if (keep) {
+    uint32_t id = ids[i];
+    const uint32_t j = C.nn[i];
+    if (j > i && j < count && C.nn[j] == i) {  // merges with a higher place
+      const uint32_t other = ids[j], merged = atomicAdd(&C.counters[kNextId], 1u);
+      const float4 a = C.lo[id], b = C.lo[other], c = C.hi[id], d = C.hi[other];
+      C.lo[merged] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z),
+                                 __uint_as_float(__float_as_uint(a.w) + __float_as_uint(b.w)));
+      C.hi[merged] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z),
+                                 __uint_as_float(max(__float_as_uint(c.w), __float_as_uint(d.w)) + 1u));
+      C.child[merged - C.n] = make_uint2(id, other);
+      id = merged;
+    }
+    out[at] = id;
+  }
+  if (blockIdx.x == (count - 1) / kClusterThreads && threadIdx.x == kClusterThreads - 1)
+    C.counters[kCount + (turn ^ 1)] = at + (keep ? 1u : 0u);
+}
+
+// One level of the wide tree: its nodes w, each over the binary cluster
+// cluster_of[w]. A node starts from its cluster and opens the largest
+// until it has four (clusters of more than three triangles before smaller
+// ones); what is left of up to three triangles becomes a leaf. The next level's
+// nodes are appended to cluster_of. Boxes are widened by 1e-6 of their
+// coordinates: the traversal's p * i + o rounds by less.
+__device__ __forceinline__ void widen(const Clusters& C, uint32_t* cluster_of, uint32_t w, const uint32_t* order,
+                                      const float4* tri, WideNode* wide, float4* leaf) {
+  uint32_t c[4] = {cluster_of[w], 0u, 0u, 0u};
+  int k = 1;
+  while (k < 4) {
+    int pick = -1;
+    bool pick_large = false;
+    float pick_area = 0.0f;
+    for (int x = 0; x < k; ++x) {
+      const float4 lo = C.lo[c[x]];
+      const uint32_t tris = __float_as_uint(lo.w);
+      if (tris < 2) continue;
+      const bool large = tris > kLeafTris;
+      const float area = half_area(lo, C.hi[c[x]]);
+      if (pick < 0 || (large && !pick_large) || (large == pick_large && area > pick_area)) {
+        pick = x;
+        pick_large = large;
+        pick_area = area;
+      }
+    }
+    if (pick < 0) break;
+    const uint2 ch = C.child[c[pick] - C.n];
+    c[pick] = ch.x;
+    c[k++] = ch.y;
+  }
+  uint32_t nodes = 0, leaf_tris = 0;
+  for (int s = 0; s < k; ++s) {
+    const uint32_t tris = __float_as_uint(C.lo[c[s]].w);
+    if (tris > kLeafTris) ++nodes; else leaf_tris += tris;
+  }
+  WideNode N = {};
+  N.node0 = atomicAdd(&C.counters[kWide], nodes);
+  N.tri0 = atomicAdd(&C.counters[kLeafs], leaf_tris);
+  uint32_t node_at = N.node0, tri_at = N.tri0;
+  float* plane = reinterpret_cast<float*>(N.plane);  // [6][4]
+  const float inf = __int_as_float(0x7F800000);
+  for (int s = 0; s < 4; ++s) {
+    if (s >= k) {
+      for (int a = 0; a < 3; ++a) {
+        plane[8 * a + s] = inf;
+        plane[8 * a + 4 + s] = -inf;
+      }
+      continue;
+    }
+    const float4 lo = C.lo[c[s]], hi = C.hi[c[s]];
+    const float l3[3] = {lo.x, lo.y, lo.z}, h3[3] = {hi.x, hi.y, hi.z};
+    for (int a = 0; a < 3; ++a) {
+      const float pad = fmaxf(fabsf(l3[a]), fabsf(h3[a])) * 1e-6f;
+      plane[8 * a + s] = l3[a] - pad;
+      plane[8 * a + 4 + s] = h3[a] + pad;
+    }
+    const uint32_t tris = __float_as_uint(lo.w);
+    if (tris > kLeafTris) {
+      N.contents |= 1u << (24 + s);
+      cluster_of[node_at++] = c[s];
+      continue;
+    }
+    N.contents |= ((1u << tris) - 1u) << (3 * s);
+    // the cluster's triangles (at most three): left child first
+    uint32_t todo[3] = {c[s], 0u, 0u};
+    for (int sp = 1; sp > 0;) {
+      const uint32_t x = todo[--sp];
+      if (x >= C.n) {
+        const uint2 ch = C.child[x - C.n];
+        todo[sp++] = ch.y;
+        todo[sp++] = ch.x;
+        continue;
+      }
+      const uint32_t t = order[x];
+      const float4 v0 = tri[size_t(t) * 3], v1 = tri[size_t(t) * 3 + 1], v2 = tri[size_t(t) * 3 + 2];
+      float4* out = leaf + size_t(tri_at++) * 3;
+      out[0] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(t));
+      out[1] = make_float4(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z, 0.0f);
+      out[2] = make_float4(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z, 0.0f);
+    }
+  }
+  wide[w] = N;
+}
+
+__global__ void __launch_bounds__(128) widen_kernel(Clusters C, uint32_t* cluster_of, int level, const uint32_t* order,
+                                                    const float4* tri, WideNode* wide, float4* leaf) {
+  const uint32_t end = C.counters[kLevelEnd + level + 1];
+  for (uint32_t w = C.counters[kLevelEnd + level] + blockIdx.x * 128u + threadIdx.x; w < end; w += gridDim.x * 128u)
+    widen(C, cluster_of, w, order, tri, wide, leaf);
+}
+
 float srgb_to_linear(int i) {
   const double c = i / 255.0;
   return static_cast<float>(c <= 0.04045 ? c / 12.92 : std::pow((c + 0.055) / 1.055, 2.4));
@@ -878,38 +1229,52 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
   cudaGetDevice(&B->device);
   B->tris = n;
   B->nodes = n > 1 ? n - 1 : 0;
-  const size_t tri_bytes = size_t(n) * 3 * sizeof(float4), node_bytes = size_t(B->nodes) * 2 * sizeof(uint4);
-  if ((e = cudaMalloc(&B->block, tri_bytes + node_bytes + 256)) != cudaSuccess) {
+  // Each wide node but the root is over more than kLeafTris triangles and so has
+  // more than kLeafTris children (or four): with c children a node, N nodes and
+  // at most n leaves, c N <= N - 1 + n.
+  static_assert(kLeafTris >= 1 && kLeafTris <= 3, "at most three triangles a slot, four slots");
+  const size_t nn = n, max_wide = nn / kLeafTris + 2;
+  const size_t tri_bytes = nn * 3 * sizeof(float4), guard_bytes = nn * 2 * sizeof(float4);
+  if ((e = cudaMalloc(&B->block, 2 * tri_bytes + guard_bytes + max_wide * sizeof(WideNode) + 256)) != cudaSuccess) {
     delete B;
     return st(e);
   }
-  float4* tri = static_cast<float4*>(B->block);
-  uint4* node = reinterpret_cast<uint4*>(static_cast<uint8_t*>(B->block) + tri_bytes);
+  uint8_t* const block = static_cast<uint8_t*>(B->block);
+  WideNode* wide = reinterpret_cast<WideNode*>(block);
+  float4* tri = reinterpret_cast<float4*>(block + max_wide * sizeof(WideNode));
+  float4* guard = tri + 3 * nn;
+  float4* leaf = guard + 2 * nn;
   B->tri = tri;
-  B->node = node;
-  // scratch for the build
-  uint32_t *d_first = nullptr, *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr, *parent = nullptr,
-           *visits = nullptr, *box = nullptr;
-  float* cent = nullptr;
-  void* tmp = nullptr;
-  size_t tmp_bytes = 0;
-  auto cleanup = [&]() {
-    cudaFree(d_first); cudaFree(keys); cudaFree(vals); cudaFree(keys2); cudaFree(vals2);
-    cudaFree(parent); cudaFree(visits); cudaFree(box); cudaFree(cent); cudaFree(tmp);
-  };
+  B->guard = guard;
+  B->leaf = leaf;
+  B->wide = wide;
   if (n > 0) {
-    const size_t nn = n;
-    if ((e = cudaMalloc(&d_first, (ni + 1) * 4)) == cudaSuccess && (e = cudaMalloc(&keys, nn * 4)) == cudaSuccess &&
-        (e = cudaMalloc(&vals, nn * 4)) == cudaSuccess && (e = cudaMalloc(&keys2, nn * 4)) == cudaSuccess &&
-        (e = cudaMalloc(&vals2, nn * 4)) == cudaSuccess && (e = cudaMalloc(&parent, (2 * nn) * 4)) == cudaSuccess &&
-        (e = cudaMalloc(&visits, nn * 4 + 4)) == cudaSuccess && (e = cudaMalloc(&box, 64)) == cudaSuccess &&
-        (e = cudaMalloc(&cent, nn * 12)) == cudaSuccess)
-      e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, vals, vals2, static_cast<int>(n));
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes ? tmp_bytes : 16);
+    // scratch for the build: one allocation, carved below
+    size_t tmp_bytes = 0, at = 0;
+    uint32_t* const none = nullptr;
+    e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, none, none, none, none, static_cast<int>(n));
+    auto carve = [&](size_t bytes) {
+      const size_t o = at;
+      at += (bytes + 255) & ~size_t(255);
+      return o;
+    };
+    const size_t o_lo = carve(2 * nn * 16), o_hi = carve(2 * nn * 16), o_child = carve(nn * 8), o_node = carve(nn * 32),
+                 o_cent = carve(nn * 12), o_keys = carve(nn * 4), o_vals = carve(nn * 4), o_keys2 = carve(nn * 4),
+                 o_vals2 = carve(nn * 4), o_parent = carve(2 * nn * 4), o_visits = carve(nn * 4 + 4),
+                 o_kept = carve((nn / kClusterThreads + 1) * 4), o_first = carve((ni + 1) * 4), o_box = carve(64), o_count = carve(kCounters * 4),
+                 o_tmp = carve(tmp_bytes ? tmp_bytes : 16);
+    uint8_t* m = nullptr;
+    if (e == cudaSuccess) e = cudaMalloc(&m, at);
+    auto u32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(m + o); };
+    uint32_t *keys = u32(o_keys), *vals = u32(o_vals), *keys2 = u32(o_keys2), *vals2 = u32(o_vals2),
+             *parent = u32(o_parent), *visits = u32(o_visits), *d_first = u32(o_first), *box = u32(o_box);
+    float* cent = reinterpret_cast<float*>(m + o_cent);
+    uint4* node = reinterpret_cast<uint4*>(m + o_node);
     if (e == cudaSuccess) e = cudaMemcpy(d_first, first.data(), (ni + 1) * 4, cudaMemcpyHostToDevice);
-    uint32_t box_init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-    if (e == cudaSuccess) e = cudaMemcpy(box, box_init, 24, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(box + 8, 0, 4);  // the bad-index flag
+    const uint32_t box_init[9] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u};  // centroid bounds; bad flag
+    const uint32_t count_init[kLevelEnd + 2] = {n, n, 0u, 1u, 0u, 0u, 1u};
+    if (e == cudaSuccess) e = cudaMemcpy(box, box_init, sizeof(box_init), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m + o_count, count_init, sizeof(count_init), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(visits, 0, nn * 4 + 4);
     BuildArgs A{*scene, d_ranges, d_first, ni, n};
     const uint32_t blocks = (n + 255) / 256;
@@ -920,20 +1285,57 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
       e = cudaGetLastError();
     }
     if (e == cudaSuccess)
-      e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, vals2, static_cast<int>(n), 0, 30);
-    if (e == cudaSuccess && n > 1) {
-      hierarchy_kernel<<<(n - 1 + 255) / 256, 256>>>(keys2, vals2, static_cast<int>(n), node, parent);
-      refit_kernel<<<blocks, 256>>>(tri, static_cast<int>(n), node, parent, visits);
+      e = cub::DeviceRadixSort::SortPairs(m + o_tmp, tmp_bytes, keys, keys2, vals, vals2, static_cast<int>(n), 0, 30);
+    if (e == cudaSuccess) {
+      if (n > 1) {
+        hierarchy_kernel<<<(n - 1 + 255) / 256, 256>>>(keys2, vals2, static_cast<int>(n), node, parent);
+        refit_kernel<<<blocks, 256>>>(tri, static_cast<int>(n), node, parent, visits);
+      }
+      guard_kernel<<<blocks, 256>>>(static_cast<int>(n), node, parent, guard);
       e = cudaGetLastError();
+    }
+    // the clustering, from the triangles in Morton order (vals2) to one cluster
+    Clusters C{reinterpret_cast<float4*>(m + o_lo), reinterpret_cast<float4*>(m + o_hi),
+               reinterpret_cast<uint2*>(m + o_child), parent, u32(o_kept), u32(o_count), n};
+    uint32_t *ids = keys, *next = vals;
+    if (e == cudaSuccess) cluster_init_kernel<<<blocks, 256>>>(C, vals2, guard, tri, ids);
+    // (batches of passes and levels: each read-back of a count costs as much as a pass)
+    for (uint32_t count = n; count > 1 && e == cudaSuccess;) {
+      const uint32_t g = (count + kClusterThreads - 1) / kClusterThreads, before = count;
+      for (int pass = 0; pass < 8; ++pass) {
+        nearest_kernel<<<g, kClusterThreads>>>(C, ids, pass & 1);
+        kept_kernel<<<g, kClusterThreads>>>(C, pass & 1);
+        merge_kernel<<<g, kClusterThreads>>>(C, ids, next, pass & 1);
+        std::swap(ids, next);
+      }
+      if ((e = cudaGetLastError()) == cudaSuccess)
+        e = cudaMemcpy(&count, C.counters + kCount, 4, cudaMemcpyDeviceToHost);
+      if (e == cudaSuccess && (count == 0 || count >= before)) e = cudaErrorUnknown;  // every pass merges a pair
+    }
+    // the wide tree, one launch per level; node 0 is over the last cluster
+    uint32_t* cluster_of = keys2;
+    int levels = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(cluster_of, ids, 4, cudaMemcpyDeviceToDevice);
+    bool done = false;
+    while (!done && e == cudaSuccess && levels <= kStack) {
+      for (int l = 0; l < 4 && levels <= kStack; ++l, ++levels) {
+        widen_kernel<<<1216, 128>>>(C, cluster_of, levels, vals2, tri, wide, leaf);
+        e = cudaMemcpyAsync(C.counters + kLevelEnd + levels + 2, C.counters + kWide, 4, cudaMemcpyDeviceToDevice);
+      }
+      if (e == cudaSuccess) e = cudaGetLastError();
+      uint32_t ends[2];
+      if (e == cudaSuccess)
+        e = cudaMemcpy(ends, C.counters + kLevelEnd + levels, 8, cudaMemcpyDeviceToHost);
+      if (e == cudaSuccess) done = ends[0] == ends[1];
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     uint32_t bad = 0;
     if (e == cudaSuccess) e = cudaMemcpy(&bad, box + 8, 4, cudaMemcpyDeviceToHost);
-    cleanup();
-    if (e == cudaSuccess && bad) {
+    cudaFree(m);
+    if (e == cudaSuccess && (bad || !done)) {
       cudaFree(B->block);
       delete B;
-      return NRC_ERROR_INVALID_ARGUMENT;  // an index past the scene's buffers
+      return bad ? NRC_ERROR_INVALID_ARGUMENT : NRC_ERROR_TOO_LARGE;  // an index past the scene's buffers; see kMaxHeight
     }
   }
   if (e != cudaSuccess) {
@@ -977,7 +1379,7 @@ int nrc_path_trace(const nrc_scene* scene, const nrc_bvh* bvh, const nrc_trace_p
   TraceArgs A;
   A.sc.s = *scene;
   for (int i = 0; i < 256; ++i) A.sc.lut[i] = srgb_to_linear(i);
-  A.bvh = TriView{bvh->tri, bvh->node, bvh->tris};
+  A.bvh = TriView{bvh->tri, bvh->guard, bvh->leaf, bvh->wide, bvh->tris};
   A.p = *p;
   A.t = *t;
   dim3 grid((p->width + 7) / 8, (p->height + 7) / 8);
