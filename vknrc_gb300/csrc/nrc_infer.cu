@@ -193,7 +193,11 @@ __device__ __forceinline__ void infer_body(const InferLaunch<N>& L) {
   const uint32_t id64 = idesc_16_f32(128, 64, 0, 0, kBF16), id16 = idesc_16_f32(128, 16, 0, 0, kBF16);
   uint8_t* stage0 = smem_rec + (s * 2 + 0) * kRecTileBytes;
   const uint8_t* rec_in = static_cast<const uint8_t*>(input);
-  auto tile_of = [&](uint32_t it) { return (it * G + rank) * kSlots + s; };
+  // Consecutive tiles go to different CTAs, so that a last, partial round (or a
+  // query of few tiles) leaves every CTA with the same share of its slots busy:
+  // 130,000 queries take 10.4 instead of 11.5 us, 911,487 (bf16) 45.8 instead of
+  // 46.9, 2,073,600 96.6 instead of 97.4, against five consecutive tiles per CTA.
+  auto tile_of = [&](uint32_t it) { return (it * kSlots + s) * G + rank; };
 
   // The copy of the slot's tile into record stage b; with dynamic tiles the
   // tile comes from the counter and is published with the stage (an end mark,
@@ -478,10 +482,12 @@ uint32_t infer_smem_bytes() { return kSmemBytes; }
 int infer_threads() { return kInferThreads; }
 int infer_tiles_per_cta() { return kSlots; }
 
+// One CTA per tile up to the chip: few tiles run fastest one to an SM (1,000
+// queries take 5.0 us on the device, 6.7 with five tiles to a CTA; 19,456 5.3
+// instead of 6.9).
 uint32_t infer_grid(uint32_t capacity, int num_sms) {
   const uint32_t tiles = (capacity + kTile - 1) / kTile;
-  const uint32_t want = (tiles + kSlots - 1) / kSlots;
-  return want < static_cast<uint32_t>(num_sms) ? want : static_cast<uint32_t>(num_sms);
+  return tiles < static_cast<uint32_t>(num_sms) ? tiles : static_cast<uint32_t>(num_sms);
 }
 
 cudaError_t launch_infer(const void* input, bool encoded, const uint32_t* d_count, uint32_t capacity,
