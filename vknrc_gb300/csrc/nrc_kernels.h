@@ -152,9 +152,11 @@ cudaError_t launch_infer_many(const InferJob* jobs, int njobs, const uint32_t* g
 // One launch of the persistent trainer: up to NRC_TRAIN_BATCH_COUNT chained
 // batches, each a fused gradient pass followed by the optimizer step (mode
 // kTrainStep), or one gradient pass whose fixed-order sum is written to
-// grad_out (kGradientOnly).
+// grad_out (kGradientOnly), or one gradient pass that leaves the CTAs' partial
+// sums for apply_kernel and does the prepare pass (kPartials).
 constexpr int kTrainStep = 0;
 constexpr int kGradientOnly = 1;
+constexpr int kPartials = 2;
 
 struct TrainBatch {
   const nrc_train_record* records;
@@ -220,7 +222,9 @@ cudaError_t launch_loss_rows(const float* pred, const float* target, const uint3
 uint32_t train_smem_bytes();
 uint32_t train_grid(const TrainParams& p, int max_ctas);
 // The grid barrier counter p.sync[0] and exit counter p.sync[1] must be zero
-// before the first launch on them; every launch leaves them at zero.
+// before the first launch on them; every launch leaves them at zero. A single
+// step runs as two ordinary launches, bit for bit the one cooperative launch's
+// result (see launch_train_step).
 cudaError_t launch_train(const TrainParams& p, const CUtensorMap* wmap, int max_ctas, cudaStream_t stream);
 // One cooperative launch training njobs caches, group_size[j] CTAs for job j
 // (1 .. 160 each, sum <= CTAs resident at one per SM). Jobs must not share a

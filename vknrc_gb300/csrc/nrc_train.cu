@@ -213,6 +213,16 @@ __device__ __forceinline__ bool grid_sync(uint32_t* counter, uint32_t target, ui
   return *reinterpret_cast<volatile uint32_t*>(sync_ok) != 0;
 }
 
+// The step state after one more step (nrc_train_prepare.comp:20-27).
+__device__ __forceinline__ nrc_optimizer_state advance(nrc_optimizer_state st, const TrainParams& P) {
+  st.t += 1;
+  st.beta1_t *= P.beta1;
+  st.beta2_t *= P.beta2;
+  st.alpha_t_1 = st.alpha_t;
+  st.alpha_t *= P.ema_alpha;
+  return st;
+}
+
 // One launch trains up to N caches: CTAs [group_start[j], group_start[j+1])
 // form cache j's group, which runs the whole schedule below on its own (its own
 // grid barrier, partial slots and parameter slices). With N = 1 the group is the
@@ -266,6 +276,8 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
   // fills the SMs this grid leaves free); dependents that read this launch's
   // results wait for its completion in their own griddepcontrol.wait.
   griddep_launch_dependents();
+  // A lone gradient pass starts its weight copy before it knows its records.
+  if (P.mode == kPartials && threadIdx.x == 0) stage_weights_tma(smem_w, &wmap, &B->w_full);
 
   // This CTA's slice [c0, c1) of float4 gradient columns in the optimizer phase;
   // its optimizer entries stay in shared memory for the whole launch (only this
@@ -292,11 +304,12 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
   const uint32_t tmem = __shfl_sync(0xffffffffu, B->tmem_base, 0);
   float* const my_partial = P.partials + static_cast<size_t>(rank) * kParams;
   nrc_optimizer_state st = B->st;  // advanced per batch in every CTA alike
-  if (P.mode == kTrainStep && rank == 0 && threadIdx.x == 0) {
+  if (P.mode != kGradientOnly && rank == 0 && threadIdx.x == 0) {
     // Other CTAs read either the raw or the clamped count; both clamp to the same n.
     for (int s = 0; s < P.steps; ++s) *P.batch[s].d_count = min(B->count[s], P.batch_cap);
   }
   auto batch_records = [&](int s) { return min(min(B->count[s], P.batch_cap), P.batch[s].capacity); };
+  if (P.mode == kPartials && rank == 0 && threadIdx.x == 0 && batch_records(0) > 0) *P.state = advance(*P.state, P);
   auto tiles_of = [&](uint32_t num_tiles) { return rank < num_tiles ? (num_tiles - rank + G - 1) / G : 0u; };
 
   // Role state that persists across the batches (mbarrier phases).
@@ -413,14 +426,13 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
     const uint32_t n = batch_records(step);
     const uint32_t num_tiles = (n + kTile - 1) / kTile;
     const uint32_t my_tiles = tiles_of(num_tiles);
-    if (P.mode == kTrainStep && n > 0) {  // the optimizer phase updates exactly when records were processed
-      st.t += 1;
-      st.beta1_t *= P.beta1;
-      st.beta2_t *= P.beta2;
-      st.alpha_t_1 = st.alpha_t;
-      st.alpha_t *= P.ema_alpha;
+    // the optimizer phase updates exactly when records were processed
+    if (P.mode == kTrainStep && n > 0) st = advance(st, P);
+    if (P.mode != kPartials) {
+      if (threadIdx.x == 0 && my_tiles > 0) stage_weights_tma(smem_w, &wmap, &B->w_full);
+    } else if (warp == 0 && my_tiles == 0) {  // landed before the CTA leaves
+      ok = warp_all(mbar_wait(&B->w_full, 0, kWaitLimitNs));
     }
-    if (threadIdx.x == 0 && my_tiles > 0) stage_weights_tma(smem_w, &wmap, &B->w_full);
 
     if (warp == 0) {
       // ---------------------------------------------------- MMA issuer --
@@ -593,6 +605,10 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
     if (my_tiles > 0) ++wloads;
     if (!ok && lane == 0) atomicOr(P.err, kErrTimeout);
     ok = __syncthreads_and(ok) != 0;  // one decision per CTA from here on
+    if (P.mode == kPartials) {
+      if (!ok && threadIdx.x == 0) atomicOr(P.err, kErrPartials);
+      break;
+    }
 
     // The record stages are free again: the next batch's first tiles land
     // during the grid barrier and the optimizer phase.
@@ -718,7 +734,7 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
   // The group's barrier counter (sync[0]) starts every launch at zero: the last
   // CTA of the group to get here, when every CTA has left its barrier waits,
   // resets it and the exit counter (sync[1]).
-  if (threadIdx.x == 0) {
+  if (P.mode != kPartials && threadIdx.x == 0) {
     __threadfence();
     B->sync_ok = atomicAdd(P.sync + 1, 1u) == G - 1 ? 1u : 0u;
     if (B->sync_ok != 0u) {
@@ -740,6 +756,68 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_steps_kernel(const __g
   train_body<N, kBF16, false>(L);
 }
 
+// One optimizer step from the partial gradients of a kPartials launch of `ctas`
+// CTAs: four threads per float4 column sum every fourth partial and combine as
+// (s0 + s1) + (s2 + s3), the fused launch's order, and thread `part` updates
+// parameter 4 * column + part. A warp's load takes a whole 128-byte line of each
+// of four partials.
+struct ApplyParams {
+  const float* partials;
+  const uint32_t* d_count;  // clamped by the gradient pass
+  const nrc_optimizer_state* state;
+  nrc_optimizer_entry* entries;
+  uint16_t *w16, *use16;  // use16: null unless the step writes it
+  const uint32_t* err;
+  uint32_t capacity, batch_cap, ctas;
+  AdamHyper hp;
+};
+// 20 loads in flight a thread: more would take registers (104 here) that let its
+// CTAs wait beside the gradient pass's (38 loads: 24.7 against 18.4 us at 16,384
+// records, in a graph).
+constexpr int kApplyThreads = 128, kApplyLoads = 20;
+
+template <bool kBF16>
+__global__ void __launch_bounds__(kApplyThreads) apply_kernel(const __grid_constant__ ApplyParams A) {
+  griddep_launch_dependents();
+  griddep_wait();  // the partials, the step state and the clamped count
+  const uint32_t part = threadIdx.x & 3u, col = blockIdx.x * (kApplyThreads / 4) + (threadIdx.x >> 2);
+  const bool in = col < static_cast<uint32_t>(kCols4);
+  const uint32_t k = 4 * col + part;
+  const float4 v = __ldcg(reinterpret_cast<const float4*>(A.entries + (in ? k : 0u)));
+  const nrc_optimizer_state st = *A.state;
+  const uint32_t err = *A.err, n = min(min(*A.d_count, A.batch_cap), A.capacity);
+  if (n == 0 || (err & kErrPartials) != 0u) return;
+  const uint32_t active = min(A.ctas, (n + kTile - 1) / kTile);
+  nrc_optimizer_entry e{v.x, v.y, v.z, v.w};
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4* p = reinterpret_cast<const float4*>(A.partials) + (in ? col : 0u);
+  for (uint32_t r0 = part; r0 < active; r0 += 4 * kApplyLoads) {
+    float4 g[kApplyLoads];
+#pragma unroll
+    for (int j = 0; j < kApplyLoads; ++j)
+      if (r0 + 4 * j < active) g[j] = __ldcg(p + static_cast<size_t>(r0 + 4 * j) * kCols4);
+#pragma unroll
+    for (int j = 0; j < kApplyLoads; ++j)
+      if (r0 + 4 * j < active) {
+        acc.x += g[j].x;
+        acc.y += g[j].y;
+        acc.z += g[j].z;
+        acc.w += g[j].w;
+      }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int off = 1; off <= 2; off <<= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
+    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, off);
+    acc.w += __shfl_xor_sync(0xffffffffu, acc.w, off);
+  }
+  if (!in) return;
+  const float gsum = part == 0 ? acc.x : part == 1 ? acc.y : part == 2 ? acc.z : acc.w;
+  adam_one<kBF16>(static_cast<int>(k), gsum, n, st, A.hp, e, A.entries, A.w16, A.use16);
+}
+
 // The batched training over a launch table in global memory.
 __global__ void __launch_bounds__(kTrainThreads, 1)
     train_table_kernel(const TrainLaunch<kMaxTrainJobs>* __restrict__ L) {
@@ -747,23 +825,23 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 }
 
 template <int N>
-cudaError_t launch(const TrainLaunch<N>& L, uint32_t grid, cudaStream_t stream, bool bf16) {
-  // Cooperative (the grid barrier needs every CTA resident) and a programmatic
+cudaError_t launch(const TrainLaunch<N>& L, uint32_t grid, cudaStream_t stream, bool bf16, bool cooperative = true) {
+  // Cooperative where the grid barrier needs every CTA resident, and a programmatic
   // dependent of the preceding kernel: the launch is issued before that kernel
   // ends, its CTAs take SMs as the preceding kernel's CTAs leave, and
   // griddepcontrol.wait holds them until it has completed.
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeCooperative;
+  attr[1].val.cooperative = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kTrainThreads);
   cfg.dynamicSmemBytes = kTrainSmemBytes;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = cooperative ? 2 : 1;
   return bf16 ? cudaLaunchKernelEx(&cfg, train_steps_kernel<N, true>, L)
               : cudaLaunchKernelEx(&cfg, train_steps_kernel<N, false>, L);
 }
@@ -791,6 +869,44 @@ uint32_t train_grid(const TrainParams&, int max_ctas) {
   return static_cast<uint32_t>(max_ctas) < kMaxTrainCtas ? static_cast<uint32_t>(max_ctas) : kMaxTrainCtas;
 }
 
+// One step as two ordinary launches, the gradient pass and the optimizer step,
+// the second a programmatic dependent of the first: its small CTAs wait beside
+// the gradient's. In place of a grid barrier there is a kernel boundary, and no
+// cooperative launch, which on a stream (not in a graph) costs 2-3 us a call:
+// 1,000 records take 14.4 instead of 18.6 us, 16,384 19.4 instead of 20.7, 65,536 35.6
+// instead of 36.1 (L is the caller's launch, for the whole grid).
+// More steps stay one launch: there the barriers overlap the next batch's first
+// tile, and four chained steps of 16,384 took 78 us this way against 66.
+cudaError_t launch_train_step(TrainLaunch<1>& L, uint32_t grid, cudaStream_t stream) {
+  TrainParams& p = L.job[0].p;
+  const TrainBatch& b = p.batch[0];
+  p.mode = kPartials;
+  const cudaError_t e = launch(L, grid, stream, p.bf16 != 0, false);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((kCols4 * 4 + kApplyThreads - 1) / kApplyThreads);
+  cfg.blockDim = dim3(kApplyThreads);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  ApplyParams A;
+  A.partials = p.partials;
+  A.d_count = b.d_count;
+  A.state = p.state;
+  A.entries = p.entries;
+  A.w16 = reinterpret_cast<uint16_t*>(p.w16);
+  A.use16 = b.write_use ? reinterpret_cast<uint16_t*>(p.use16) : nullptr;
+  A.err = p.err;
+  A.capacity = b.capacity;
+  A.batch_cap = p.batch_cap;
+  A.ctas = grid;
+  A.hp = AdamHyper{p.lr, p.beta1, p.beta2, p.eps, p.ema_alpha, p.loss_scale, p.use_ema};
+  return p.bf16 != 0 ? cudaLaunchKernelEx(&cfg, apply_kernel<true>, A) : cudaLaunchKernelEx(&cfg, apply_kernel<false>, A);
+}
+
 cudaError_t launch_train(const TrainParams& p, const CUtensorMap* wmap, int max_ctas, cudaStream_t stream) {
   if (p.steps < 1 || p.steps > NRC_TRAIN_BATCH_COUNT) return cudaErrorInvalidValue;
   const uint32_t grid = train_grid(p, max_ctas);
@@ -801,6 +917,7 @@ cudaError_t launch_train(const TrainParams& p, const CUtensorMap* wmap, int max_
   L.group_start[0] = 0;
   L.group_start[1] = grid;
   L.njobs = 1;
+  if (p.steps == 1 && p.mode == kTrainStep && p.join.src == nullptr) return launch_train_step(L, grid, stream);
   return launch(L, grid, stream, p.bf16 != 0);
 }
 
