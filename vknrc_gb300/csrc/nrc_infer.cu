@@ -12,9 +12,18 @@
 //     fp16) back into the A columns for the next layer;
 //   - kSlots independent 128-record tiles are in flight per CTA, one warpgroup
 //     each (thread <-> record row, warp k of a slot reads TMEM lanes 32k..+31).
-//     Every slot issues its own MMAs from its first warp (converged, one lane
+//     Every slot issues its own MMAs from one of its warps (converged, one lane
 //     elected): a single issuing thread is bounded by its issue rate, several
 //     issuing warps keep the tensor pipe busy while other slots convert.
+// Bound by the latency of each slot's chain (encode, then six rounds of barrier,
+// MMA and epilogue), which the other slots' instructions on the same scheduler
+// lengthen; five slots are what tensor memory holds. Measured at 2,073,600 records
+// (fp16 / FP8 at 3,686,400): 97.0 / 190.8 us with the first warp of every slot
+// issuing, all five on one scheduler; 94.5 / 186.0 with the issuing warps spread over
+// the four; 90.0 / 175.9 with the layer loop unrolled and the output layer apart;
+// 88.5 / 169.8 with the record copies on another warp, after the slot's first A
+// operand is handed over. The FP8 form gains no more because E4M3 adds a multiply
+// per value to a chain that the tensor pipe does not bound.
 #include <mutex>
 
 #include "nrc_common.cuh"
@@ -183,8 +192,10 @@ __device__ __forceinline__ void infer_body(const InferLaunch<N>& L) {
   const int s = warp >> 2;  // slot
   const int q = warp & 3;   // TMEM lane quadrant of this warp
   const int row = q * 32 + lane;
-  const bool issuer = q == 0;
-  const bool leader = q == 0 && lane == 0;
+  // The slot's MMAs and its record copies are issued by warps of different
+  // schedulers (warp % 4), and those of the slots by different ones.
+  const bool issuer = q == (s & 3);
+  const bool leader = q == ((s + 2) & 3) && lane == 0;
   SlotBars& B = bars[s];
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t a_col = tmem + s * kSlotCols, d_col = a_col + 32;  // lane-0 addresses of the slot
@@ -275,16 +286,21 @@ __device__ __forceinline__ void infer_body(const InferLaunch<N>& L) {
       }
       // the stage may be refilled once all 128 threads have read it
       mbar_arrive(&B.rec_empty[b]);
+      // layer-0 A operand: 16-bit features, column pair (2j, 2j+1) in word j (the
+      // halves stored as they are made), or E4M3 features 4j..4j+3 in word j; each
+      // store after the warp has reconverged
       if (kF8) {
         encode_input_e4m3(r, inv_sx0, e);
+        __syncwarp();
+        tmem_st16(a_col + lane_off, e);
       } else {
-        encode_input<kBF16>(r, e);
-      }
-      if (leader && (dyn || tile_of(it + 2) < num_tiles)) {
-        if (!mbar_wait(&B.rec_empty[b], (it >> 1) & 1, kWaitLimitNs))
-          atomicOr(err, kErrTimeout);
-        else
-          fill_stage(b, tile_of(it + 2));
+        encode_half0<kBF16>(r, e);
+        __syncwarp();
+        tmem_st16_async(a_col + lane_off, e);
+        encode_half1<kBF16>(r, e + 16);
+        __syncwarp();
+        tmem_st16_async(a_col + lane_off + 16, e + 16);
+        tmem_wait_st();
       }
     } else {
       const uint16_t* enc_in = static_cast<const uint16_t*>(input);
@@ -303,48 +319,60 @@ __device__ __forceinline__ void infer_body(const InferLaunch<N>& L) {
         for (int c = 0; c < 32; ++c) e[c] = 0u;
       }
     }
-    __syncwarp();  // reconverge before the warp-collective TMEM store
-    // layer-0 A operand: 16-bit features, column pair (2j, 2j+1) in word j, or
-    // E4M3 features 4j..4j+3 in word j
-    if (kF8)
-      tmem_st16(a_col + lane_off, e);
-    else
+    if (kEncoded) {
+      __syncwarp();
       tmem_st32(a_col + lane_off, e);
+    }
     tc_fence_before();
     arrive_warp(&B.a_ready);
-#pragma unroll 1
-    for (int l = 0; l < 6; ++l) {
-      if (issuer) {
-        ok = warp_all(mbar_wait(&B.a_ready, ph_a, kWaitLimitNs));
-        if (ok) {
-          ph_a ^= 1u;  // counts issued layers; ph_d counts observed completions
-          tc_fence_after();
-          if (elect_one()) {
-            const uint64_t wl = wdesc + static_cast<uint64_t>(l * 512);
-            if (kF8) {
-              mma_ts_f8(d_col, a_col + 0, wl + 0, l < 5 ? id64 : id16, 0u);
-              mma_ts_f8(d_col, a_col + 8, wl + 2, l < 5 ? id64 : id16, 1u);
-            } else {
-              issue_layer(d_col, a_col, wl, l < 5 ? id64 : id16);
-            }
-            mma_commit(&B.d_ready);
-          }
-          __syncwarp();
-        }
+    if (!kEncoded) {  // the stage's next tile
+      const uint32_t b = it & 1;
+      if (leader && (dyn || tile_of(it + 2) < num_tiles)) {
+        if (!mbar_wait(&B.rec_empty[b], (it >> 1) & 1, kWaitLimitNs))
+          atomicOr(err, kErrTimeout);
+        else
+          fill_stage(b, tile_of(it + 2));
       }
-      // load the destination word while the output layer's MMAs run
-      if (kScatter && l == 5 && row < static_cast<int>(rows_valid)) qdst = __ldg(Q.dst + grow);
-      const float cl = kF8 ? J.fp8->c[l] : 1.0f;  // the layer's scale constant (FP8 query)
+      __syncwarp();
+    }
+    // Layer l's MMAs, once its A operand is in TMEM (the slot's issuing warp).
+    auto issue = [&](int l, uint32_t id) {
+      if (!issuer) return;
+      ok = warp_all(mbar_wait(&B.a_ready, ph_a, kWaitLimitNs));
+      if (!ok) return;
+      ph_a ^= 1u;  // counts issued layers; ph_d counts observed completions
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t wl = wdesc + static_cast<uint64_t>(l * 512);
+        if (kF8) {
+          mma_ts_f8(d_col, a_col + 0, wl + 0, id, 0u);
+          mma_ts_f8(d_col, a_col + 8, wl + 2, id, 1u);
+        } else {
+          issue_layer(d_col, a_col, wl, id);
+        }
+        mma_commit(&B.d_ready);
+      }
+      __syncwarp();
+    };
+    // The accumulator is ready; false on a time-out.
+    auto wait_d = [&]() -> bool {
       ok = ok && warp_all(mbar_wait(&B.d_ready, ph_d, kWaitLimitNs));
-      if (!ok) break;
+      if (!ok) return false;
       ph_d ^= 1u;
       tc_fence_after();
-      if (kF8 && l < 5) {
-        // all 64 accumulator columns in one load and one wait, packed in place
-        // (word j from values 4j..4j+3, j <= 4j); the scale multiplies two
-        // lanes per instruction (IEEE-rounded like __fmul_rn each)
-        uint32_t v[64];
-        tmem_ld64(d_col + lane_off, v);
+      return true;
+    };
+#pragma unroll
+    for (int l = 0; l < 5; ++l) {
+      issue(l, id64);
+      const float cl = kF8 ? J.fp8->c[l] : 1.0f;  // the layer's scale constant (FP8 query)
+      if (!wait_d()) break;
+      // all 64 accumulator columns in one load and one wait, converted in place
+      uint32_t v[64];
+      tmem_ld64(d_col + lane_off, v);
+      if (kF8) {
+        // word j from values 4j..4j+3, j <= 4j; the scale multiplies two lanes per
+        // instruction (IEEE-rounded like __fmul_rn each)
         const uint64_t c2 = f32x2(cl, cl);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -354,34 +382,38 @@ __device__ __forceinline__ void infer_body(const InferLaunch<N>& L) {
           v[j] = pack4_relu_e4m3(a0, a1, a2, a3);
         }
         tmem_st16(a_col + lane_off, *reinterpret_cast<uint32_t(*)[16]>(v));
-        tc_fence_before();
-        arrive_warp(&B.a_ready);
-      } else if (l < 5) {
-        // all 64 accumulator columns in one load and one wait, converted in place
-        uint32_t v[64];
-        tmem_ld64(d_col + lane_off, v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = pack2_relu<kBF16>(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-        tmem_st32(a_col + lane_off, *reinterpret_cast<uint32_t(*)[32]>(v));
-        tc_fence_before();
-        arrive_warp(&B.a_ready);
       } else {
-        uint32_t o4[4];
-        tmem_ld4(d_col + lane_off, o4);
-        if (row < static_cast<int>(rows_valid)) {
-          if (Q.out != nullptr) {
-            float* dst = Q.out + grow * 3;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const float v = kF8 ? __fmul_rn(__uint_as_float(o4[c]), cl) : __uint_as_float(o4[c]);
-              dst[c] = Q.clamp ? fmaxf(v, 0.0f) : v;
-            }
-          }
-          if (kScatter)
-            scatter_query(Q, qdst, fmaxf(__uint_as_float(o4[0]), 0.0f), fmaxf(__uint_as_float(o4[1]), 0.0f),
-                          fmaxf(__uint_as_float(o4[2]), 0.0f));
+        for (int j = 0; j < 16; ++j) v[j] = pack2_relu<kBF16>(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+        tmem_st16_async(a_col + lane_off, v);
+#pragma unroll
+        for (int j = 16; j < 32; ++j) v[j] = pack2_relu<kBF16>(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+        tmem_st16_async(a_col + lane_off + 16, v + 16);
+        tmem_wait_st();
+      }
+      tc_fence_before();
+      arrive_warp(&B.a_ready);
+    }
+    if (!ok) break;
+    issue(5, id16);
+    // load the destination word while the output layer's MMAs run
+    if (kScatter && row < static_cast<int>(rows_valid)) qdst = __ldg(Q.dst + grow);
+    const float cl = kF8 ? J.fp8->c[5] : 1.0f;
+    if (!wait_d()) break;
+    uint32_t o4[4];
+    tmem_ld4(d_col + lane_off, o4);
+    if (row < static_cast<int>(rows_valid)) {
+      if (Q.out != nullptr) {
+        float* dst = Q.out + grow * 3;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float v = kF8 ? __fmul_rn(__uint_as_float(o4[c]), cl) : __uint_as_float(o4[c]);
+          dst[c] = Q.clamp ? fmaxf(v, 0.0f) : v;
         }
       }
+      if (kScatter)
+        scatter_query(Q, qdst, fmaxf(__uint_as_float(o4[0]), 0.0f), fmaxf(__uint_as_float(o4[1]), 0.0f),
+                      fmaxf(__uint_as_float(o4[2]), 0.0f));
     }
   }
   if (!ok && lane == 0) atomicOr(err, kErrTimeout);
