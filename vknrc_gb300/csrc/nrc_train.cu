@@ -82,7 +82,9 @@ struct TrainBars {
   uint64_t rec_full[2];
   uint64_t rec_empty[2];
   uint64_t a_ready;    // 8 arrivals (one per epilogue warp): the next A operand is in TMEM
-  uint64_t g_ready;    // 8 arrivals: a gradient's shared-memory rows (weight-gradient operand) are written
+  uint64_t g_ready[2];  // 8 arrivals: the rows of gradient buffer 0 / 1 (weight-gradient operand) are written.
+                        // One barrier each: the MMA warp may still wait for one gradient's rows when the
+                        // epilogue, which needs only dA, completes the next one's.
   uint64_t d_ready;    // MMA commit: scratch accumulator ready
   uint64_t tile_done;  // MMA commit after the tile's last weight-gradient MMA
   uint64_t drain;
@@ -258,7 +260,8 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
     mbar_init(&B->rec_empty[0], kEpiThreads);
     mbar_init(&B->rec_empty[1], kEpiThreads);
     mbar_init(&B->a_ready, kEpiWarps);
-    mbar_init(&B->g_ready, kEpiWarps);
+    mbar_init(&B->g_ready[0], kEpiWarps);
+    mbar_init(&B->g_ready[1], kEpiWarps);
     mbar_init(&B->d_ready, 1);
     mbar_init(&B->tile_done, 1);
     mbar_init(&B->drain, 1);
@@ -322,7 +325,7 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
   const uint32_t a_lane = lane_base + kACol + 16 * h;
   const uint32_t d_lane = lane_base + kDCol + 32 * h;
   uint32_t ph_a = 0, ph_d = 0;  // MMA warp / epilogue d_ready phases
-  uint32_t ph_g = 0;            // MMA warp: g_ready phase
+  uint32_t ph_g = 0;            // MMA warp: g_ready phases (bit b: barrier b)
   uint32_t ct = 0;              // tiles this CTA has processed over all batches
   uint32_t wloads = 0;          // weight loads issued to this CTA
   uint32_t barriers = 0;        // grid barriers passed
@@ -350,10 +353,10 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
   };
   // Every shared-memory operand row this thread wrote so far (activations, the
   // gradient just stored) is visible to the tensor core: one arrival per warp.
-  auto release_smem = [&]() {
+  auto release_smem = [&](int b) {
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&B->g_ready);
+    if (lane == 0) mbar_arrive(&B->g_ready[b]);
   };
   // Epilogue warps: records of the CTA's tile `it` -> target, and the encoded
   // input act_0 in shared memory and TMEM, published to the MMA warp.
@@ -490,9 +493,9 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
           }
           // the weight gradient reads g_{l+1}'s shared-memory rows (and act_l),
           // written after the TMEM copy that dA_l reads
-          ok = warp_all(mbar_wait(&B->g_ready, ph_g, kWaitLimitNs));
+          ok = warp_all(mbar_wait(&B->g_ready[(5 - l) & 1], (ph_g >> ((5 - l) & 1)) & 1u, kWaitLimitNs));
           if (!ok) break;
-          ph_g ^= 1u;
+          ph_g ^= 1u << ((5 - l) & 1);
           tc_fence_after();
           if (elect_one()) {
             // dW_l += g^T act_l   (M = 64 outputs, N = 64 inputs, K = 128 records);
@@ -573,7 +576,7 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
           }
           release_tmem();
           store_half(gbuf, row, h, gw);  // read by dW_5
-          release_smem();                // (with act_0 .. act_5)
+          release_smem(0);               // (with act_0 .. act_5)
         }
         // backward: g_l = fp16((g_{l+1} W_l) masked by act_l > 0), l = 5..1
         for (int l = 5; l >= 1; --l) {
@@ -587,7 +590,7 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
           tmem_st16(a_lane, gw);
           release_tmem();
           store_half(gbuf + ((6 - l) & 1) * kActBytes, row, h, gw);  // read by dW_{l-1}
-          release_smem();
+          release_smem((6 - l) & 1);
           // dA_l completing means dW_{l+1} (issued before it) is complete too;
           // on the CTA's last tile it is final: write it out while the chain goes on.
           if (last && l <= 4) drain_dw(lane_base, l + 1, q, h, lane, my_partial);
