@@ -424,14 +424,20 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 
 // Closest triangle along the ray in [tmin, tmax]; equal distances go to the lower
 // triangle index. Returns the triangle index or -1. Kept out of line, which
-// keeps its registers apart from the shading's (inlined: 1.73 against
-// 1.68 ms).
+// keeps its registers apart from the shading's (inlined: 1.73 against 1.68 ms).
 // The lanes that call together step together: each iteration is one node for
 // every lane with a node to visit, or one triangle test for every lane with
-// triangles pending, chosen so that steps run with many lanes (left to diverge
-// freely, the loops ran with 6 lanes per instruction). A lane goes on visiting
-// nodes until the triangles of two nodes are pending.
-__device__ __noinline__ int trace_closest(const TriView& B, Ray r, float tmin, float tmax, float& bt_out, float& bu,
+// triangles pending, chosen so that steps run with many lanes. A lane goes on
+// visiting nodes until the triangles of two nodes are pending.
+// Bound by instruction issue at the warp's lane count (ncu, 587,534 triangles,
+// 8-bounce paths at 960 x 540: issue slots 62%, ALU pipe 62%, 12.4 of 32 lanes; L1
+// wavefronts 48%): 12 nodes and 4.7 triangles a ray. That launch takes 1.67 ms; the
+// binary radix tree with freely diverging lanes took 3.18 ms (6 lanes), this loop
+// over eight-wide nodes of 8-bit planes 2.25, over four-wide ones 1.88 (unpacking
+// the bytes loads the half-rate ALU pipe more than fp32 planes load L1). Lanes that
+// finish early and shade while the others go on walking made it slower (1.95 ms):
+// the shading, a third of the instructions, then runs more often with fewer lanes.
+__device__ __noinline__ int trace_closest(const TriView B, Ray r, float tmin, float tmax, float& bt_out, float& bu,
                                           float& bv) {
   if (B.tris == 0) return -1;
   const float ix = fabsf(r.d.x) > 1e-20f ? 1.0f / r.d.x : copysignf(1e20f, r.d.x);
@@ -728,7 +734,7 @@ __device__ __forceinline__ Result trace_path(const TraceArgs& A, const float* lu
 // consecutive threads (4 rows), the warp standing in for the subgroup.
 // 16 blocks of 64 threads per SM (64 registers): 12 blocks without spills and
 // with the traversal inlined measured slower (1.85 against 1.68 ms for 8-bounce
-// paths at 960 x 540, 1.83 against 1.74 ms for cache paths at 1920 x 1080; 2.72 ms
+// paths at 960 x 540, 1.83 against 1.70 ms for cache paths at 1920 x 1080; 2.72 ms
 // over the binary tree).
 __global__ void __launch_bounds__(64, 16) path_trace_kernel(const __grid_constant__ TraceArgs A) {
   extern __shared__ float lut_s[];
