@@ -120,18 +120,11 @@ __device__ void t_sincos_turns(float u, float& so, float& co) {
   co = q == 0 ? cs : q == 1 ? -sn : q == 2 ? -cs : sn;
 }
 
-// atan on [0, inf): 1/z above 1 (pi/2 - atan), then atan z = pi/6 + atan((z sqrt3 - 1) / (z + sqrt3))
-// above tan(pi/12), then the odd Taylor series to z^13.
-__device__ float t_atan_pos(float z) {
-  bool inv = false, shift = false;
-  if (z > 1.0f) {
-    z = 1.0f / z;
-    inv = true;
-  }
-  if (z > 0.267949194f) {
-    z = (z * 1.73205081f - 1.0f) / (z + 1.73205081f);
-    shift = true;
-  }
+// atan on [0, 1]: atan z = pi/6 + atan((z sqrt3 - 1) / (z + sqrt3)) above tan(pi/12),
+// then the odd Taylor series to z^13.
+__device__ float t_atan_unit(float z) {
+  const bool shift = z > 0.267949194f;
+  if (shift) z = (z * 1.73205081f - 1.0f) / (z + 1.73205081f);
   const float z2 = z * z;
   float p = 1.0f / 13.0f;
   p = fmaf(p, z2, -1.0f / 11.0f);
@@ -140,16 +133,16 @@ __device__ float t_atan_pos(float z) {
   p = fmaf(p, z2, 1.0f / 5.0f);
   p = fmaf(p, z2, -1.0f / 3.0f);
   p = fmaf(p, z2, 1.0f);
-  float a = z * p;
-  if (shift) a = a + 0.523598790f;
-  if (inv) a = 1.57079637f - a;
-  return a;
+  const float a = z * p;
+  return shift ? a + 0.523598790f : a;
 }
 
 __device__ float t_atan2(float y, float x) {
   const float ax = fabsf(x), ay = fabsf(y);
   if (ax == 0.0f && ay == 0.0f) return 0.0f;
-  float a = ay <= ax ? t_atan_pos(ay / ax) : 1.57079637f - t_atan_pos(ax / ay);
+  const bool low = ay <= ax;
+  float a = t_atan_unit((low ? ay : ax) / (low ? ax : ay));
+  if (!low) a = 1.57079637f - a;
   if (x < 0.0f) a = kPi - a;
   return y < 0.0f ? -a : a;
 }
@@ -220,54 +213,60 @@ __device__ V3 align_dir(V3 n, V3 d) {
   const V3 v = cross(n, u);
   return add(add(scale(u, d.x), scale(v, d.y)), scale(n, d.z));
 }
-__device__ V3 sample_cosine(V3 n, Rng& rng) {  // Sample.glsl:13-20 (direction only)
-  const float u1 = rng.next(), u2 = rng.next();
-  const float r = sqrtf(u1);
-  float s, c;
-  t_sincos_turns(u2, s, c);
-  return align_dir(n, v3(r * c, r * s, sqrtf(1.0f - u1)));
-}
-__device__ V3 ct_eval(const Brdf& b, V3 l, V3 v, V3 n) {
+// The BRDF's value and the sampling density of l (CookTorranceEval and
+// CookTorrancePdf), which share the half vector, its cosines and, unless n.h is
+// clamped, the distribution. `w` is ct_spec_prob(b).
+__device__ V3 ct_eval_pdf(const Brdf& b, V3 l, V3 v, V3 n, float w, float& pdf) {
   const V3 h = normalize(add(l, v));
-  const float n_dot_h = fmaxf(dot(n, h), 1e-8f);
-  const float v_dot_h = fmaxf(dot(v, h), 1e-8f), l_dot_h = v_dot_h;
-  const float n_dot_l = fminf(fmaxf(dot(n, l), 1e-8f), 1.0f - 1e-8f);
+  const float nl = dot(n, l), nh = dot(n, h), vh = dot(v, h);
+  const float n_dot_h = fmaxf(nh, 1e-8f);
+  const float v_dot_h = fmaxf(vh, 1e-8f), l_dot_h = v_dot_h;
+  const float n_dot_l = fminf(fmaxf(nl, 1e-8f), 1.0f - 1e-8f);
   const float n_dot_v = fminf(fmaxf(dot(n, v), 1e-8f), 1.0f - 1e-8f);
   const float a = b.roughness, a2 = a * a;
   const float G = walter_g1(v_dot_h, n_dot_v, a2) * walter_g1(l_dot_h, n_dot_l, a2);
   const float D = beckmann_d(n_dot_h, a2);
   const float F = schlick(v_dot_h, b.ior);
+  pdf = 0.0f;
+  if (!(nl < 0.0f)) {
+    const float p_h = (nh == n_dot_h ? D : beckmann_d(nh, a2)) * nh;
+    const float p_ct = p_h / (4.0f * vh);
+    const float p_l = nl / kPi;
+    pdf = p_l * (1.0f - w) + p_ct * w;  // mix(p_lambert, p_cook_torrance, w)
+  }
   // specular * D * G * F / (4 n.l n.v), left to right per channel; diffuse / pi
   const V3 spec = divs(scale(scale(scale(b.specular, D), G), F), 4.0f * n_dot_l * n_dot_v);
   return add(divs(b.diffuse, kPi), spec);
 }
-__device__ float ct_pdf(const Brdf& b, V3 l, V3 v, V3 n) {
-  const float n_dot_l = dot(l, n);
-  if (n_dot_l < 0.0f) return 0.0f;
-  const V3 h = normalize(add(l, v));
-  const float a = b.roughness;
-  const float p_h = beckmann_d(dot(n, h), a * a) * dot(n, h);
-  const float p_ct = p_h / (4.0f * dot(v, h));
-  const float p_l = n_dot_l / kPi;
-  const float w = ct_spec_prob(b);
-  return p_l * (1.0f - w) + p_ct * w;  // mix(p_lambert, p_cook_torrance, w)
-}
-// CookTorranceSample: returns the incident direction; pdf via ct_pdf.
-__device__ V3 ct_sample(const Brdf& b, V3 v, V3 n, Rng& rng) {
-  const float a = b.roughness, a2 = a * a;
-  float tan2 = -a2 * t_log(1.0f - rng.next());
-  if (tan2 != tan2) tan2 = 0.0f;
-  const float n_dot_h = sqrtf(1.0f / (1.0f + tan2));
+// CookTorranceSample: returns the incident direction; pdf via ct_eval_pdf. The half
+// vector of the specular lobe and the cosine-weighted direction of the diffuse one
+// (Sample.glsl:13-20) are the same steps from a radius, an angle and a height, so
+// the lanes of either lobe take them together.
+__device__ V3 ct_sample(const Brdf& b, V3 v, V3 n, float w, Rng& rng) {
+  const float u1 = rng.next(), u2 = rng.next();
+  const bool diffuse = rng.next() > w;
+  float r, z, turn;
+  if (diffuse) {
+    const float c1 = rng.next();
+    turn = rng.next();
+    r = sqrtf(c1);
+    z = sqrtf(1.0f - c1);
+  } else {
+    const float a = b.roughness, a2 = a * a;
+    float tan2 = -a2 * t_log(1.0f - u1);
+    if (tan2 != tan2) tan2 = 0.0f;
+    z = sqrtf(1.0f / (1.0f + tan2));
+    r = sqrtf(1.0f - z * z);
+    turn = u2;
+  }
   float s, c;
-  t_sincos_turns(rng.next(), s, c);
-  const float r = sqrtf(1.0f - n_dot_h * n_dot_h);
-  V3 h = align_dir(n, v3(r * c, r * s, n_dot_h));
-  if (dot(v, h) < 0.0f) h = neg(h);
+  t_sincos_turns(turn, s, c);
+  const V3 d = align_dir(n, v3(r * c, r * s, z));
+  if (diffuse) return d;
+  const V3 h = dot(v, d) < 0.0f ? neg(d) : d;
   // reflect(-v, h) = -v - 2 dot(h, -v) h
   const V3 iv = neg(v);
-  V3 l = sub(iv, scale(h, 2.0f * dot(h, iv)));
-  if (rng.next() > ct_spec_prob(b)) l = sample_cosine(n, rng);
-  return l;
+  return sub(iv, scale(h, 2.0f * dot(h, iv)));
 }
 
 __device__ __forceinline__ V3 normalize_rgb(V3 c) {  // NormalizeRGB, path_tracer.comp:147
@@ -295,6 +294,7 @@ __device__ V3 scene_vertex(const nrc_scene& S, uint32_t inst, uint32_t prim, int
 __device__ float lerpf(float a, float b, float t) { return a + (b - a) * t; }
 
 __device__ uint32_t wrap_idx(float f, uint32_t n) {
+  if ((n & (n - 1u)) == 0u) return static_cast<uint32_t>(static_cast<int>(f)) & (n - 1u);  // the same, f being integral
   const float nf = static_cast<float>(n);
   int r = static_cast<int>(f - nf * floorf(f / nf));
   if (r < 0) r += static_cast<int>(n);
@@ -576,9 +576,10 @@ struct Step {  // BRDFStepInfo
 __device__ Step brdf_step(const Hit& h, Ray ray, Rng& rng) {  // BRDFStep, path_tracer.comp:167-186
   Brdf b{h.diffuse, h.specular, fmaxf(h.roughness, 0.001f), fmaxf(h.ior, 1.5f)};
   const V3 v = neg(ray.d);
-  const V3 dir = ct_sample(b, v, h.normal, rng);
-  const float pdf = ct_pdf(b, dir, v, h.normal);
-  const V3 f = ct_eval(b, dir, v, h.normal);
+  const float w = ct_spec_prob(b);
+  const V3 dir = ct_sample(b, v, h.normal, w, rng);
+  float pdf;
+  const V3 f = ct_eval_pdf(b, dir, v, h.normal, w, pdf);
   const float cosine = fabsf(dot(h.normal, dir));
   Step s;
   s.color = normalize_rgb(divs(scale(f, cosine), pdf));  // brdf * cosine / pdf
@@ -735,7 +736,10 @@ __device__ __forceinline__ Result trace_path(const TraceArgs& A, const float* lu
 // 16 blocks of 64 threads per SM (64 registers): 12 blocks without spills and
 // with the traversal inlined measured slower (1.85 against 1.68 ms for 8-bounce
 // paths at 960 x 540, 1.83 against 1.70 ms for cache paths at 1920 x 1080; 2.72 ms
-// over the binary tree).
+// over the binary tree). The shading's length counts twice, in issue slots and in
+// instruction cache misses: one atan for either octant, one half vector and
+// distribution for the BRDF's value and density and one direction for both lobes
+// took the same launches from 1.66 and 1.70 to 1.60 and 1.55 ms.
 __global__ void __launch_bounds__(64, 16) path_trace_kernel(const __grid_constant__ TraceArgs A) {
   extern __shared__ float lut_s[];
   for (int i = threadIdx.y * 8 + threadIdx.x; i < 256; i += 64) lut_s[i] = A.sc.lut[i];
