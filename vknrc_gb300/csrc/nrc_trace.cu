@@ -1010,9 +1010,47 @@ __global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const flo
   ids[i] = i;
 }
 
-// Equal areas choose the nearer place, then the pair that starts at an even
-// place, so that runs of equal boxes pair up. Clusters kMaxHeight high count as
-// infinitely far: what is left then pairs by place, which bounds the tree's height.
+// The place that place i of `count` chooses; lo and hi hold the boxes, place i's at
+// index `at`. Equal areas choose the nearer place, then the pair that starts at an
+// even place, then the lower place, so that runs of equal boxes pair up and some
+// pair always chooses each other: of the pairs with the least area, distance and
+// parity, the lowest does. Clusters kMaxHeight high count as infinitely far: what is
+// left then pairs by place, which bounds the tree's height.
+__device__ __forceinline__ uint32_t nearest_place(const float4* lo, const float4* hi, int at, int i, int count) {
+  const float4 l = lo[at], h = hi[at];
+  float best_d = 0.0f;
+  uint32_t best_k = 0, best_j = 0xFFFFFFFFu;
+  for (int o = -kSearch; o <= kSearch; ++o) {
+    const int j = i + o;
+    if (o == 0 || j < 0 || j >= count) continue;
+    const float4 a = lo[at + o], b = hi[at + o];
+    float d = half_area(make_float4(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z), 0.0f),
+                        make_float4(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z), 0.0f));
+    if (max(__float_as_uint(h.w), __float_as_uint(b.w)) >= kMaxHeight) d = __int_as_float(0x7F800000);
+    const uint32_t key = 2u * static_cast<uint32_t>(abs(o)) + (static_cast<uint32_t>(min(i, j)) & 1u);
+    if (best_j == 0xFFFFFFFFu || d < best_d || (d == best_d && key < best_k)) {
+      best_d = d;
+      best_k = key;
+      best_j = static_cast<uint32_t>(j);
+    }
+  }
+  return best_j;
+}
+
+// Merges clusters `id` and `other` (their boxes given): the new id, its box in lo, hi.
+__device__ __forceinline__ uint32_t merge_clusters(const Clusters& C, uint32_t id, uint32_t other, float4& lo, float4& hi,
+                                                   float4 olo, float4 ohi) {
+  const uint32_t merged = atomicAdd(&C.counters[kNextId], 1u);
+  lo = make_float4(fminf(lo.x, olo.x), fminf(lo.y, olo.y), fminf(lo.z, olo.z),
+                   __uint_as_float(__float_as_uint(lo.w) + __float_as_uint(olo.w)));
+  hi = make_float4(fmaxf(hi.x, ohi.x), fmaxf(hi.y, ohi.y), fmaxf(hi.z, ohi.z),
+                   __uint_as_float(max(__float_as_uint(hi.w), __float_as_uint(ohi.w)) + 1u));
+  C.lo[merged] = lo;
+  C.hi[merged] = hi;
+  C.child[merged - C.n] = make_uint2(id, other);
+  return merged;
+}
+
 // The passes run in batches, grids sized by the count before the batch: the
 // count of a pass is in counters[kCount + turn].
 __global__ void __launch_bounds__(kClusterThreads) nearest_kernel(Clusters C, const uint32_t* ids, int turn) {
@@ -1028,26 +1066,8 @@ __global__ void __launch_bounds__(kClusterThreads) nearest_kernel(Clusters C, co
     }
   }
   __syncthreads();
-  const int i = base + kSearch + static_cast<int>(threadIdx.x);
-  if (i >= static_cast<int>(count)) return;
-  const float4 lo = slo[threadIdx.x + kSearch], hi = shi[threadIdx.x + kSearch];
-  float best_d = 0.0f;
-  uint32_t best_k = 0, best_j = 0xFFFFFFFFu;
-  for (int o = -kSearch; o <= kSearch; ++o) {
-    const int j = i + o;
-    if (o == 0 || j < 0 || j >= static_cast<int>(count)) continue;
-    const float4 a = slo[threadIdx.x + kSearch + o], b = shi[threadIdx.x + kSearch + o];
-    float d = half_area(make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), 0.0f),
-                        make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), 0.0f));
-    if (max(__float_as_uint(hi.w), __float_as_uint(b.w)) >= kMaxHeight) d = __int_as_float(0x7F800000);
-    const uint32_t key = 2u * static_cast<uint32_t>(abs(o)) + (static_cast<uint32_t>(min(i, j)) & 1u);
-    if (best_j == 0xFFFFFFFFu || d < best_d || (d == best_d && key < best_k)) {
-      best_d = d;
-      best_k = key;
-      best_j = static_cast<uint32_t>(j);
-    }
-  }
-  C.nn[i] = best_j;
+  const int at = static_cast<int>(threadIdx.x) + kSearch, i = base + at;
+  if (i < static_cast<int>(count)) C.nn[i] = nearest_place(slo, shi, at, i, static_cast<int>(count));
 }
 
 // Place i survives unless it merges into a lower place.
@@ -1092,19 +1112,64 @@ __global__ void __launch_bounds__(kClusterThreads) merge_kernel(Clusters C, cons
     uint32_t id = ids[i];
     const uint32_t j = C.nn[i];
     if (j > i && j < count && C.nn[j] == i) {  // merges with a higher place
-      const uint32_t other = ids[j], merged = atomicAdd(&C.counters[kNextId], 1u);
-      const float4 a = C.lo[id], b = C.lo[other], c = C.hi[id], d = C.hi[other];
-      C.lo[merged] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z),
-                                 __uint_as_float(__float_as_uint(a.w) + __float_as_uint(b.w)));
-      C.hi[merged] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z),
-                                 __uint_as_float(max(__float_as_uint(c.w), __float_as_uint(d.w)) + 1u));
-      C.child[merged - C.n] = make_uint2(id, other);
-      id = merged;
+      const uint32_t other = ids[j];
+      float4 lo = C.lo[id], hi = C.hi[id];
+      id = merge_clusters(C, id, other, lo, hi, C.lo[other], C.hi[other]);
     }
     out[at] = id;
   }
   if (blockIdx.x == (count - 1) / kClusterThreads && threadIdx.x == kClusterThreads - 1)
     C.counters[kCount + (turn ^ 1)] = at + (keep ? 1u : 0u);
+}
+
+// The last passes, from at most kFinishThreads clusters to one, in one block: as
+// launches they are small and many (about 30 of a tree's 60 passes). The last
+// cluster's id goes to *root.
+constexpr int kFinishThreads = 512;
+__global__ void __launch_bounds__(kFinishThreads) finish_kernel(Clusters C, const uint32_t* ids, uint32_t* root) {
+  __shared__ float4 slo[kFinishThreads], shi[kFinishThreads];
+  __shared__ uint32_t sid[kFinishThreads], snn[kFinishThreads], warps[kFinishThreads / 32];
+  uint32_t count = C.counters[kCount];
+  const uint32_t i = threadIdx.x, lane = i & 31u, warp = i >> 5;
+  if (i < count) {
+    sid[i] = ids[i];
+    slo[i] = C.lo[ids[i]];
+    shi[i] = C.hi[ids[i]];
+  }
+  __syncthreads();
+  for (int pass = 0; count > 1 && pass < kFinishThreads; ++pass) {  // every pass merges a pair: see nearest_place
+    if (i < count) snn[i] = nearest_place(slo, shi, static_cast<int>(i), static_cast<int>(i), static_cast<int>(count));
+    __syncthreads();
+    const uint32_t j = i < count ? snn[i] : 0u;
+    const bool mutual = i < count && snn[j] == i, keep = i < count && !(mutual && j < i);
+    float4 lo = {}, hi = {};
+    uint32_t id = 0;
+    if (keep) {
+      id = sid[i];
+      lo = slo[i];
+      hi = shi[i];
+      if (mutual) id = merge_clusters(C, id, sid[j], lo, hi, slo[j], shi[j]);
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) warps[warp] = __popc(m);
+    __syncthreads();
+    uint32_t at = __popc(m & ((1u << lane) - 1u)), total = 0;
+    for (uint32_t w = 0; w < kFinishThreads / 32; ++w) {
+      if (w < warp) at += warps[w];
+      total += warps[w];
+    }
+    if (keep) {
+      sid[at] = id;
+      slo[at] = lo;
+      shi[at] = hi;
+    }
+    count = total;
+    __syncthreads();
+  }
+  if (i == 0) {
+    *root = sid[0];
+    C.counters[kCount] = count;
+  }
 }
 
 // One level of the wide tree: its nodes w, each over the binary cluster
@@ -1310,7 +1375,7 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
     uint32_t *ids = keys, *next = vals;
     if (e == cudaSuccess) cluster_init_kernel<<<blocks, 256>>>(C, vals2, guard, tri, ids);
     // (batches of passes and levels: each read-back of a count costs as much as a pass)
-    for (uint32_t count = n; count > 1 && e == cudaSuccess;) {
+    for (uint32_t count = n; count > kFinishThreads && e == cudaSuccess;) {
       const uint32_t g = (count + kClusterThreads - 1) / kClusterThreads, before = count;
       for (int pass = 0; pass < 8; ++pass) {
         nearest_kernel<<<g, kClusterThreads>>>(C, ids, pass & 1);
@@ -1322,10 +1387,10 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
         e = cudaMemcpy(&count, C.counters + kCount, 4, cudaMemcpyDeviceToHost);
       if (e == cudaSuccess && (count == 0 || count >= before)) e = cudaErrorUnknown;  // every pass merges a pair
     }
-    // the wide tree, one launch per level; node 0 is over the last cluster
     uint32_t* cluster_of = keys2;
+    if (e == cudaSuccess) finish_kernel<<<1, kFinishThreads>>>(C, ids, cluster_of);
+    // the wide tree, one launch per level; node 0 is over the last cluster
     int levels = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cluster_of, ids, 4, cudaMemcpyDeviceToDevice);
     bool done = false;
     while (!done && e == cudaSuccess && levels <= kStack) {
       for (int l = 0; l < 4 && levels <= kStack; ++l, ++levels) {
@@ -1339,8 +1404,10 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
       if (e == cudaSuccess) done = ends[0] == ends[1];
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    uint32_t bad = 0;
+    uint32_t bad = 0, left = 1;
     if (e == cudaSuccess) e = cudaMemcpy(&bad, box + 8, 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&left, C.counters + kCount, 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && left != 1) e = cudaErrorUnknown;
     cudaFree(m);
     if (e == cudaSuccess && (bad || !done)) {
       cudaFree(B->block);
