@@ -685,13 +685,18 @@ int ensure_eval_ws(nrc_context* c, uint32_t capacity) {
   return NRC_OK;
 }
 
+// Checks a call's packed eval records and grows their workspace.
+int eval_ws(nrc_context* c, const nrc_eval_record* rec, const uint32_t* d_count, uint32_t capacity) {
+  if (rec == nullptr || d_count == nullptr) return NRC_ERROR_INVALID_ARGUMENT;
+  if (reinterpret_cast<uintptr_t>(rec) & 3u) return NRC_ERROR_MISALIGNED;
+  return ensure_eval_ws(c, capacity);
+}
+
 // Unpacks min(*d_count, capacity) packed eval records (and, with dst, their
 // destination words) into the context's workspace.
 int unpack_eval_ws(nrc_context* c, const nrc_scene* scene, const nrc_eval_record* rec, const uint32_t* d_count,
                    uint32_t capacity, bool dst, cudaStream_t st) {
-  if (rec == nullptr || d_count == nullptr) return NRC_ERROR_INVALID_ARGUMENT;
-  if (reinterpret_cast<uintptr_t>(rec) & 3u) return NRC_ERROR_MISALIGNED;
-  int s = ensure_eval_ws(c, capacity);
+  int s = eval_ws(c, rec, d_count, capacity);
   if (s != NRC_OK) return s;
   return from_cuda(nrc::launch_unpack(*scene, prim_rows(scene), mat_rows(scene), false, rec, d_count, capacity,
                                       c->eval_ws, dst ? c->eval_dst_ws : nullptr, c->num_sms, st));
@@ -716,24 +721,27 @@ int ensure_train_ws(nrc_context* c, uint32_t capacity) {
   return NRC_OK;
 }
 
-// Unpacks the frame's packed train batches into the workspace; ws[b] receives
-// batch b's array.
-int unpack_train_ws(nrc_context* c, const nrc_scene* scene, const nrc_packed_train_record* const* rec,
-                    uint32_t* const* counts, uint32_t capacity, const nrc_train_record** ws, cudaStream_t st) {
+// Checks a frame's packed train batches and grows their workspace; ws[b]
+// receives batch b's array.
+int train_ws(nrc_context* c, const nrc_packed_train_record* const* rec, uint32_t* const* counts, uint32_t capacity,
+             nrc_train_record** ws) {
   for (int b = 0; b < NRC_TRAIN_BATCH_COUNT; ++b) {
     if (counts[b] == nullptr || (capacity > 0 && rec[b] == nullptr)) return NRC_ERROR_INVALID_ARGUMENT;
     if (rec[b] != nullptr && (reinterpret_cast<uintptr_t>(rec[b]) & 3u)) return NRC_ERROR_MISALIGNED;
   }
   int s = ensure_train_ws(c, capacity > 0 ? capacity : 1);
   if (s != NRC_OK) return s;
-  nrc_train_record* out[NRC_TRAIN_BATCH_COUNT];
-  for (int b = 0; b < NRC_TRAIN_BATCH_COUNT; ++b) {
-    out[b] = c->train_ws + size_t(b) * c->train_ws_cap;
-    ws[b] = out[b];
-  }
-  if (capacity == 0) return NRC_OK;
+  for (int b = 0; b < NRC_TRAIN_BATCH_COUNT; ++b) ws[b] = c->train_ws + size_t(b) * c->train_ws_cap;
+  return NRC_OK;
+}
+
+// Unpacks the frame's packed train batches into the workspace.
+int unpack_train_ws(nrc_context* c, const nrc_scene* scene, const nrc_packed_train_record* const* rec,
+                    uint32_t* const* counts, uint32_t capacity, nrc_train_record** ws, cudaStream_t st) {
+  int s = train_ws(c, rec, counts, capacity, ws);
+  if (s != NRC_OK || capacity == 0) return s;
   return from_cuda(nrc::launch_unpack_train_batches(*scene, prim_rows(scene), mat_rows(scene), rec, counts, capacity,
-                                                    out, NRC_TRAIN_BATCH_COUNT, c->num_sms, st));
+                                                    ws, NRC_TRAIN_BATCH_COUNT, c->num_sms, st));
 }
 
 }  // namespace
@@ -805,7 +813,7 @@ int nrc_frame_scatter_packed(nrc_context* c, const nrc_scene* scene, const nrc_e
   if (s != NRC_OK) return s;
   const nrc_packed_train_record* prec[NRC_TRAIN_BATCH_COUNT];
   for (int b = 0; b < NRC_TRAIN_BATCH_COUNT; ++b) prec[b] = targets->train_records[b];
-  const nrc_train_record* ws[NRC_TRAIN_BATCH_COUNT];
+  nrc_train_record* ws[NRC_TRAIN_BATCH_COUNT];
   if ((s = unpack_train_ws(c, scene, prec, train_counts, cap, ws, static_cast<cudaStream_t>(stream))) != NRC_OK)
     return s;
   return nrc_train_batches(c, ws, train_counts, cap, NRC_TRAIN_BATCH_COUNT, 1, stream);
@@ -819,14 +827,18 @@ int nrc_frame_packed(nrc_context* c, const nrc_scene* scene, const nrc_eval_reco
   if (s != NRC_OK) return s;
   if ((s = scene_check_impl(scene)) != NRC_OK) return s;
   if (train_rec == nullptr || train_counts == nullptr) return NRC_ERROR_INVALID_ARGUMENT;
-  const nrc_train_record* ws[NRC_TRAIN_BATCH_COUNT];
-  if ((s = unpack_train_ws(c, scene, train_rec, train_counts, train_capacity, ws, static_cast<cudaStream_t>(stream))) !=
-      NRC_OK)
-    return s;
-  if (eval_capacity > 0 &&
-      (s = unpack_eval_ws(c, scene, eval_rec, d_eval_count, eval_capacity, false, static_cast<cudaStream_t>(stream))) !=
-          NRC_OK)
-    return s;
+  nrc_train_record* ws[NRC_TRAIN_BATCH_COUNT];
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (eval_capacity == 0) {
+    if ((s = unpack_train_ws(c, scene, train_rec, train_counts, train_capacity, ws, st)) != NRC_OK) return s;
+  } else {
+    if ((s = train_ws(c, train_rec, train_counts, train_capacity, ws)) != NRC_OK) return s;
+    if ((s = eval_ws(c, eval_rec, d_eval_count, eval_capacity)) != NRC_OK) return s;
+    if ((s = from_cuda(nrc::launch_unpack_frame(*scene, prim_rows(scene), mat_rows(scene), train_rec, train_counts,
+                                                train_capacity, ws, eval_rec, d_eval_count, eval_capacity, c->eval_ws,
+                                                c->num_sms, st))) != NRC_OK)
+      return s;
+  }
   return frame_overlapped(c, c->eval_ws, d_eval_count, eval_capacity, out, ws, train_counts, train_capacity, nullptr, nullptr,
                           stream);
 }

@@ -262,6 +262,13 @@ cudaError_t launch_unpack_train_batches(const nrc_scene& scene, const void* prim
                                        const nrc_packed_train_record* const* in, uint32_t* const* counts,
                                        uint32_t capacity, nrc_train_record* const* out, int nbatches, int num_sms,
                                        cudaStream_t stream);
+// The train records of a frame's NRC_TRAIN_BATCH_COUNT batches and its eval records (without
+// their destination words) in one launch.
+cudaError_t launch_unpack_frame(const nrc_scene& scene, const void* prim_rows, const void* mat_rows,
+                                const nrc_packed_train_record* const* train_in, uint32_t* const* train_counts,
+                                uint32_t train_capacity, nrc_train_record* const* train_out,
+                                const nrc_eval_record* in, const uint32_t* d_count, uint32_t capacity, nrc_input* out,
+                                int num_sms, cudaStream_t stream);
 cudaError_t launch_unpack(const nrc_scene& scene, const void* prim_rows, const void* mat_rows, bool train,
                           const void* in, const uint32_t* d_count, uint32_t capacity, void* out, uint32_t* out_dst,
                           int num_sms, cudaStream_t stream);

@@ -171,6 +171,35 @@ __global__ void __launch_bounds__(kUnpackThreads, kUnpackBlocksPerSM)
                               static_cast<size_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u), stride);
 }
 
+// A frame's eval records, then its train batches, in one launch. A launch of their own gave
+// the 4 x 16,384 train records of a 1080p frame a start, a nearly empty grid and an end beside
+// 2,073,600 eval records: the packed frame takes 220.4 us with both in one launch and 229.9 us
+// with two (225.7 us with the train records first: last, they are still in L2 when the
+// training starts). The warps take the train records from the last warp down, since the eval
+// records leave the last ones a 32-record group fewer, and each batch goes on where the one
+// before it ended.
+template <bool kRows>
+__global__ void __launch_bounds__(kUnpackThreads, kUnpackBlocksPerSM)
+    unpack_frame_kernel(const __grid_constant__ UnpackParams P, const __grid_constant__ UnpackBatches U,
+                        uint32_t train_capacity, const nrc_eval_record* __restrict__ in,
+                        const uint32_t* __restrict__ d_count, uint32_t capacity, nrc_input* __restrict__ out) {
+  __shared__ float lut_smem[256 * kLutCopies];
+  __shared__ uint4 stage_smem[kUnpackThreads / 32 * kStageU4<true>];
+  const float* lut = stage_lut(lut_smem, P.lut);
+  uint4* stage = stage_smem + (threadIdx.x >> 5) * kStageU4<true>;
+  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+  const size_t first = static_cast<size_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
+  unpack_range<false, kRows>(P, in, min(*d_count, capacity), reinterpret_cast<float*>(out), nullptr, stage, lut, first,
+                             stride);
+  size_t turn = stride - 32 - first;  // this warp's place among the train records of all batches
+  for (int b = 0; b < NRC_TRAIN_BATCH_COUNT; ++b) {
+    const uint32_t n = train_capacity > 0 ? min(*U.count[b], train_capacity) : 0u;
+    unpack_range<true, kRows>(P, U.in[b], n, reinterpret_cast<float*>(U.out[b]), nullptr, stage, lut, turn, stride);
+    const size_t used = (static_cast<size_t>(n) + 31) / 32 * 32 % stride;
+    turn = turn >= used ? turn - used : turn + stride - used;
+  }
+}
+
 // nrc_scene_prepare, primitive rows: the gathers of Scene.glsl:50-58 done once
 // per primitive (vertices and texcoords copied bit for bit).
 __global__ void __launch_bounds__(256) prepare_prims_kernel(const nrc_scene S, uint4* __restrict__ rows) {
@@ -307,6 +336,33 @@ cudaError_t launch_unpack(const nrc_scene& scene, const void* prim_rows, const v
     unpack_kernel<false, true><<<grid, kUnpackThreads, 0, stream>>>(p, in, d_count, capacity, out, out_dst);
   else
     unpack_kernel<false, false><<<grid, kUnpackThreads, 0, stream>>>(p, in, d_count, capacity, out, out_dst);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_unpack_frame(const nrc_scene& scene, const void* prim_rows, const void* mat_rows,
+                                const nrc_packed_train_record* const* train_in, uint32_t* const* train_counts,
+                                uint32_t train_capacity, nrc_train_record* const* train_out,
+                                const nrc_eval_record* in, const uint32_t* d_count, uint32_t capacity, nrc_input* out,
+                                int num_sms, cudaStream_t stream) {
+  const uint64_t records = uint64_t(capacity) + uint64_t(NRC_TRAIN_BATCH_COUNT) * train_capacity;
+  const uint64_t want = (records + kUnpackThreads - 1) / kUnpackThreads;
+  const uint32_t cap = static_cast<uint32_t>(num_sms) * kUnpackBlocksPerSM;  // the resident blocks
+  const uint32_t grid = want < cap ? static_cast<uint32_t>(want) : cap;
+  if (grid == 0) return cudaSuccess;
+  UnpackParams p;
+  p.scene = scene;
+  p.rows = SceneRows{static_cast<const uint4*>(prim_rows), static_cast<const uint4*>(mat_rows)};
+  p.lut = srgb_lut();
+  UnpackBatches u = {};
+  for (int b = 0; b < NRC_TRAIN_BATCH_COUNT; ++b) {
+    u.in[b] = train_in[b];
+    u.count[b] = train_counts[b];
+    u.out[b] = train_out[b];
+  }
+  if (prim_rows != nullptr)
+    unpack_frame_kernel<true><<<grid, kUnpackThreads, 0, stream>>>(p, u, train_capacity, in, d_count, capacity, out);
+  else
+    unpack_frame_kernel<false><<<grid, kUnpackThreads, 0, stream>>>(p, u, train_capacity, in, d_count, capacity, out);
   return cudaGetLastError();
 }
 
