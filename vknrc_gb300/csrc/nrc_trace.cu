@@ -400,7 +400,7 @@ __device__ __forceinline__ bool intersect(float4 a, float4 b, float4 c, Ray r, f
 // Slab test of a triangle's guard box (its parent's padded box in the binary
 // radix tree). A grazing ray's triangle test can accept a point well off the
 // triangle; a hit counts only if the ray also meets this box, so the hits do
-// not depend on how the wide tree groups and quantises its boxes (which all
+// not depend on how the wide tree groups its boxes (which all
 // contain the guard boxes).
 __device__ __forceinline__ bool guard_hit(float4 lo, float4 hi, V3 o, float ix, float iy, float iz, float tmin, float bt) {
   const float x0 = (lo.x - o.x) * ix, x1 = (hi.x - o.x) * ix;
