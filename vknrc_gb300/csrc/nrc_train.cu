@@ -158,18 +158,32 @@ __device__ __forceinline__ uint32_t relu_mask2(uint32_t g, uint32_t a) {
 
 // Write half h (32 inputs) of one layer's final weight gradient from TMEM to the
 // CTA's partial slot. M=64 accumulator layout: output row 16q+t lives in TMEM
-// lane 32q+t (t < 16), so lanes 0..15 of each warp own one output row.
-__device__ __forceinline__ void drain_dw(uint32_t lane_base, int layer, int q, int h, int lane, float* dst) {
-  const int o = q * 16 + lane;
-  const bool keep = lane < 16 && (layer < kHidden || o < kOut);
+// lane 32q+t (t < 16), so lanes 0..15 of each warp own one output row. The rows
+// pass through the warp's 2 KB of `dead`, the layer's activations, which nothing
+// reads any more (16-byte chunks swizzled by the row, free of bank conflicts), so
+// that each store instruction writes four whole 128-byte lines. Stored straight
+// from the lanes, each wrote 16 bytes of 16 lines, and the backward chain waits
+// for the drains: 4 x 16,384 records take 55.6 instead of 61.4 us (55.5 without
+// any drain beside the chain), on 38 CTAs 115.6 instead of 121.0.
+__device__ __forceinline__ void drain_dw(uint32_t lane_base, int layer, int q, int h, int lane, uint8_t* dead,
+                                         float* dst) {
+  const int rows = layer < kHidden ? 16 : min(max(kOut - q * 16, 0), 16);
+  if (rows == 0) return;
   uint32_t v[32];
   tmem_ld32(lane_base + 64 * layer + 32 * h, v);
-  if (keep) {
-    float4* g4 = reinterpret_cast<float4*>(dst + layer * kLayerElems + o * 64 + 32 * h);
+  uint4* buf = reinterpret_cast<uint4*>(dead + (h * 4 + q) * 2048);
+  if (lane < 16) {
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      g4[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
-                          __uint_as_float(v[4 * j + 3]));
+      buf[lane * 8 + (j ^ (lane & 7))] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
+  __syncwarp();
+  uint4* g4 = reinterpret_cast<uint4*>(dst + layer * kLayerElems + q * 16 * 64 + 32 * h);
+  const int c = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = 4 * i + (lane >> 3);
+    if (r < rows) g4[r * 16 + c] = buf[r * 8 + (c ^ (r & 7))];
   }
 }
 
@@ -603,15 +617,15 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
           release_smem((6 - l) & 1);
           // dA_l completing means dW_{l+1} (issued before it) is complete too;
           // on the CTA's last tile it is final: write it out while the chain goes on.
-          if (last && l <= 4) drain_dw(lane_base, l + 1, q, h, lane, my_partial);
+          if (last && l <= 4) drain_dw(lane_base, l + 1, q, h, lane, act + (l + 1) * kActBytes, my_partial);
         }
         if (!ok) break;
         if (last) {
           ok = warp_all(mbar_wait(&B->tile_done, ct & 1, kWaitLimitNs));
           if (!ok) break;
           tc_fence_after();
-          drain_dw(lane_base, 1, q, h, lane, my_partial);
-          drain_dw(lane_base, 0, q, h, lane, my_partial);
+          drain_dw(lane_base, 1, q, h, lane, act + kActBytes, my_partial);
+          drain_dw(lane_base, 0, q, h, lane, act, my_partial);
         }
       }
     }
