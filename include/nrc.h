@@ -330,7 +330,8 @@ NRC_API int nrc_loss_gradient(const float* d_pred, const float* d_target, const 
  * streams, no ordering) race; order them. d_error (may be NULL) receives the
  * device-timeout flag; when NULL a word in the scratch is used, cleared on each
  * call, which the caller cannot read: a step that hit a bounded-wait timeout
- * then still returns NRC_OK, so pass d_error to observe timeouts. Pointers that
+ * changes neither parameters nor state but still returns NRC_OK, so pass d_error
+ * to observe timeouts. Pointers that
  * are not aligned to their types (16 bytes for weights, entries and records;
  * 4 for the state, count and error words) return NRC_ERROR_MISALIGNED. */
 NRC_API int nrc_train_noalloc(uint16_t* d_weights, uint16_t* d_use_weights, nrc_optimizer_entry* d_entries,

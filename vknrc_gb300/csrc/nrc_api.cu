@@ -24,7 +24,7 @@ struct nrc_context {
   nrc_optimizer_entry* entries = nullptr;
   nrc_optimizer_state* state = nullptr;
   float* partials = nullptr;  // one weight-gradient vector per training CTA
-  uint32_t* sync = nullptr;   // grid-barrier counter of the trainer
+  uint32_t* sync = nullptr;   // barrier counters and single-step words of the trainer (64 bytes)
   uint32_t* tiles = nullptr;  // tile and exit counters of the overlapped frame's query
   uint32_t* err = nullptr;
   double* loss_acc = nullptr;

@@ -254,6 +254,5 @@ __device__ __forceinline__ void encode_input_e4m3(const float (&r)[kInFloats], f
 
 // Device-side error word bits (read back by nrc_get_error).
 constexpr uint32_t kErrTimeout = 1u;
-constexpr uint32_t kErrPartials = 2u;  // with kErrTimeout: a gradient pass gave up, its step is not applied
 
 }  // namespace nrc

@@ -178,7 +178,7 @@ struct TrainParams {
   __half* use16;
   float* partials;   // one gradient vector per CTA (grid <= the slots given)
   float* grad_out;   // kGradientOnly
-  uint32_t* sync;    // grid-barrier counter (zeroed by launch_train)
+  uint32_t* sync;    // 16 words: the grid-barrier and exit counters, then a single step's words (StepWords)
   double* loss_acc;  // optional check-path loss sum
   unsigned long long* loss_count;
   uint32_t* err;
@@ -221,10 +221,11 @@ cudaError_t launch_loss_rows(const float* pred, const float* target, const uint3
 
 uint32_t train_smem_bytes();
 uint32_t train_grid(const TrainParams& p, int max_ctas);
-// The grid barrier counter p.sync[0] and exit counter p.sync[1] must be zero
-// before the first launch on them; every launch leaves them at zero. A single
+// The words at p.sync must be zero before the first launch on them; every launch
+// leaves the grid barrier counter p.sync[0] and exit counter p.sync[1] at zero. A single
 // step runs as two ordinary launches, bit for bit the one cooperative launch's
-// result (see launch_train_step).
+// result (see launch_train_step); if a wait of its gradient pass runs out, neither
+// the parameters nor the step state change.
 cudaError_t launch_train(const TrainParams& p, const CUtensorMap* wmap, int max_ctas, cudaStream_t stream);
 // One cooperative launch training njobs caches, group_size[j] CTAs for job j
 // (1 .. 160 each, sum <= CTAs resident at one per SM). Jobs must not share a

@@ -243,6 +243,28 @@ __device__ __forceinline__ nrc_optimizer_state advance(nrc_optimizer_state st, c
   return st;
 }
 
+// A single step's two launches share these words, behind the two barrier counters of
+// `sync` (zero before the first launch on them). The gradient pass writes all but
+// `launches`, which it reads; apply_kernel writes `launches` and the cache's step
+// state, which it does not read: no launch reads a word that it also writes, so its
+// CTAs need no order among them. A CTA of the gradient pass that gives up stamps the
+// step, and then neither the parameters nor the state change. All CTAs of the apply
+// kernel read the same line at once, so they read it as two 16-byte words through L1
+// (with a load for each word from L2 1,000 records took 14.7 us, with a flag and a
+// count of the CTAs that had read it, in place of the stamp and the copy, 14.2).
+struct alignas(16) StepWords {
+  uint32_t launch;           // this step's number
+  uint32_t failed;           // the last step that gave up
+  nrc_optimizer_state next;  // the state after this step
+  uint32_t unused;
+  uint32_t launches;  // steps launched so far
+};
+constexpr int kStepWordsAt = 4;  // in sync
+__device__ __host__ __forceinline__ StepWords* step_words(uint32_t* sync) {
+  return reinterpret_cast<StepWords*>(sync + kStepWordsAt);
+}
+static_assert(kStepWordsAt * 4 + sizeof(StepWords) <= 64, "what a cache and the no-allocation step keep for `sync`");
+
 // One launch trains up to N caches: CTAs [group_start[j], group_start[j+1])
 // form cache j's group, which runs the whole schedule below on its own (its own
 // grid barrier, partial slots and parameter slices). With N = 1 the group is the
@@ -330,7 +352,11 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
     for (int s = 0; s < P.steps; ++s) *P.batch[s].d_count = min(B->count[s], P.batch_cap);
   }
   auto batch_records = [&](int s) { return min(min(B->count[s], P.batch_cap), P.batch[s].capacity); };
-  if (P.mode == kPartials && rank == 0 && threadIdx.x == 0 && batch_records(0) > 0) *P.state = advance(*P.state, P);
+  if (P.mode == kPartials && rank == 0 && threadIdx.x == 0) {
+    StepWords* const w = step_words(P.sync);
+    w->launch = w->launches + 1u;
+    w->next = advance(*P.state, P);
+  }
   auto tiles_of = [&](uint32_t num_tiles) { return rank < num_tiles ? (num_tiles - rank + G - 1) / G : 0u; };
 
   // Role state that persists across the batches (mbarrier phases).
@@ -633,7 +659,7 @@ __device__ __forceinline__ void train_body(const TrainLaunch<N>& L) {
     if (!ok && lane == 0) atomicOr(P.err, kErrTimeout);
     ok = __syncthreads_and(ok) != 0;  // one decision per CTA from here on
     if (P.mode == kPartials) {
-      if (!ok && threadIdx.x == 0) atomicOr(P.err, kErrPartials);
+      if (!ok && threadIdx.x == 0) step_words(P.sync)->failed = step_words(P.sync)->launches + 1u;
       break;
     }
 
@@ -791,13 +817,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_steps_kernel(const __g
 // (s0 + s1) + (s2 + s3), the fused launch's order, and thread `part` updates
 // parameter 4 * column + part. A warp's load takes a whole 128-byte line of each
 // of four partials.
+// The step is applied as a whole or not at all (see StepWords).
 struct ApplyParams {
   const float* partials;
   const uint32_t* d_count;  // clamped by the gradient pass
-  const nrc_optimizer_state* state;
+  nrc_optimizer_state* state;
   nrc_optimizer_entry* entries;
   uint16_t *w16, *use16;  // use16: null unless the step writes it
-  const uint32_t* err;
+  StepWords* words;
   uint32_t capacity, batch_cap, ctas;
   AdamHyper hp;
 };
@@ -814,9 +841,16 @@ __global__ void __launch_bounds__(kApplyThreads) apply_kernel(const __grid_const
   const bool in = col < static_cast<uint32_t>(kCols4);
   const uint32_t k = 4 * col + part;
   const float4 v = __ldcg(reinterpret_cast<const float4*>(A.entries + (in ? k : 0u)));
-  const nrc_optimizer_state st = *A.state;
-  const uint32_t err = *A.err, n = min(min(*A.d_count, A.batch_cap), A.capacity);
-  if (n == 0 || (err & kErrPartials) != 0u) return;
+  const uint4 w0 = *reinterpret_cast<const uint4*>(A.words), w1 = *(reinterpret_cast<const uint4*>(A.words) + 1);
+  const nrc_optimizer_state st{w0.z, __uint_as_float(w0.w), __uint_as_float(w1.x), __uint_as_float(w1.y),
+                               __uint_as_float(w1.z)};
+  const uint32_t launch = w0.x, n = min(min(*A.d_count, A.batch_cap), A.capacity);
+  const bool apply = n > 0 && w0.y != launch;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    A.words->launches = launch;
+    if (apply) *A.state = st;
+  }
+  if (!apply) return;
   const uint32_t active = min(A.ctas, (n + kTile - 1) / kTile);
   nrc_optimizer_entry e{v.x, v.y, v.z, v.w};
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -929,7 +963,7 @@ cudaError_t launch_train_step(TrainLaunch<1>& L, uint32_t grid, cudaStream_t str
   A.entries = p.entries;
   A.w16 = reinterpret_cast<uint16_t*>(p.w16);
   A.use16 = b.write_use ? reinterpret_cast<uint16_t*>(p.use16) : nullptr;
-  A.err = p.err;
+  A.words = step_words(p.sync);
   A.capacity = b.capacity;
   A.batch_cap = p.batch_cap;
   A.ctas = grid;
