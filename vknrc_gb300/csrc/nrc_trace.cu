@@ -373,8 +373,9 @@ struct TriView {
   uint32_t tris;
 };
 
-// The binary tree under the wide one is at most kMaxHeight + 31 high, and a
-// traversal stacks at most one entry per level.
+// A traversal stacks at most one entry per level of the wide tree, which has at
+// most as many as the binary tree under it is high: kMaxHeight, after which every
+// clustering pass halves what is left of fewer than 2^30 clusters.
 constexpr uint32_t kMaxHeight = 48;
 constexpr int kStack = kMaxHeight + 32;
 
@@ -959,8 +960,13 @@ __global__ void guard_kernel(int n, const uint4* node, const uint32_t* parent, f
 // larger than its neighbours (a wall beside a tessellated floor) joins late,
 // near the root, instead of stretching the boxes of everything above a small one.
 // Ids: a triangle in Morton order at [0, n), merged clusters from n on.
+// The height is bounded for every scene: once a cluster is kMaxHeight high, all later
+// passes pair the clusters by place (even with odd), which halves them, so the tree
+// gets at most 30 higher. (8,000 triangles nested in one another, of which one joins
+// the others a pass: 58 high, 131 by the search alone.)
 constexpr int kSearch = 16, kClusterThreads = 256;
 constexpr uint32_t kLeafTris = 3;
+constexpr uint32_t kNoPlace = 0xFFFFFFFFu;
 
 struct Clusters {
   float4 *lo, *hi;  // box per id; lo.w triangles below, hi.w height (as bits)
@@ -971,8 +977,9 @@ struct Clusters {
   uint32_t n;
 };
 // Counters: the next cluster id; the clusters before and after a pass (in turn);
-// wide nodes and leaf triangles so far; the wide nodes up to each level (from 0).
-constexpr int kNextId = 0, kCount = 1, kWide = 3, kLeafs = 4, kLevelEnd = 5, kCounters = kLevelEnd + kStack + 3;
+// wide nodes and leaf triangles so far; whether a cluster is kMaxHeight high; the
+// wide nodes up to each level (from 0).
+constexpr int kNextId = 0, kCount = 1, kWide = 3, kLeafs = 4, kTall = 5, kLevelEnd = 6, kCounters = kLevelEnd + kStack + 6;
 
 __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
   const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
@@ -1010,25 +1017,28 @@ __global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const flo
   ids[i] = i;
 }
 
+// The place that place i of `count` pairs with by place alone.
+__device__ __forceinline__ uint32_t paired_place(uint32_t i, uint32_t count) {
+  return (i ^ 1u) < count ? i ^ 1u : kNoPlace;
+}
+
 // The place that place i of `count` chooses; lo and hi hold the boxes, place i's at
 // index `at`. Equal areas choose the nearer place, then the pair that starts at an
 // even place, then the lower place, so that runs of equal boxes pair up and some
 // pair always chooses each other: of the pairs with the least area, distance and
-// parity, the lowest does. Clusters kMaxHeight high count as infinitely far: what is
-// left then pairs by place, which bounds the tree's height.
+// parity, the lowest does.
 __device__ __forceinline__ uint32_t nearest_place(const float4* lo, const float4* hi, int at, int i, int count) {
   const float4 l = lo[at], h = hi[at];
   float best_d = 0.0f;
-  uint32_t best_k = 0, best_j = 0xFFFFFFFFu;
+  uint32_t best_k = 0, best_j = kNoPlace;
   for (int o = -kSearch; o <= kSearch; ++o) {
     const int j = i + o;
     if (o == 0 || j < 0 || j >= count) continue;
     const float4 a = lo[at + o], b = hi[at + o];
-    float d = half_area(make_float4(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z), 0.0f),
-                        make_float4(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z), 0.0f));
-    if (max(__float_as_uint(h.w), __float_as_uint(b.w)) >= kMaxHeight) d = __int_as_float(0x7F800000);
+    const float d = half_area(make_float4(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z), 0.0f),
+                              make_float4(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z), 0.0f));
     const uint32_t key = 2u * static_cast<uint32_t>(abs(o)) + (static_cast<uint32_t>(min(i, j)) & 1u);
-    if (best_j == 0xFFFFFFFFu || d < best_d || (d == best_d && key < best_k)) {
+    if (best_j == kNoPlace || d < best_d || (d == best_d && key < best_k)) {
       best_d = d;
       best_k = key;
       best_j = static_cast<uint32_t>(j);
@@ -1038,6 +1048,7 @@ __device__ __forceinline__ uint32_t nearest_place(const float4* lo, const float4
 }
 
 // Merges clusters `id` and `other` (their boxes given): the new id, its box in lo, hi.
+// The first to be kMaxHeight high sets counters[kTall], which the next pass reads.
 __device__ __forceinline__ uint32_t merge_clusters(const Clusters& C, uint32_t id, uint32_t other, float4& lo, float4& hi,
                                                    float4 olo, float4 ohi) {
   const uint32_t merged = atomicAdd(&C.counters[kNextId], 1u);
@@ -1045,6 +1056,7 @@ __device__ __forceinline__ uint32_t merge_clusters(const Clusters& C, uint32_t i
                    __uint_as_float(__float_as_uint(lo.w) + __float_as_uint(olo.w)));
   hi = make_float4(fmaxf(hi.x, ohi.x), fmaxf(hi.y, ohi.y), fmaxf(hi.z, ohi.z),
                    __uint_as_float(max(__float_as_uint(hi.w), __float_as_uint(ohi.w)) + 1u));
+  if (__float_as_uint(hi.w) >= kMaxHeight) C.counters[kTall] = 1u;
   C.lo[merged] = lo;
   C.hi[merged] = hi;
   C.child[merged - C.n] = make_uint2(id, other);
@@ -1056,6 +1068,11 @@ __device__ __forceinline__ uint32_t merge_clusters(const Clusters& C, uint32_t i
 __global__ void __launch_bounds__(kClusterThreads) nearest_kernel(Clusters C, const uint32_t* ids, int turn) {
   const uint32_t count = C.counters[kCount + turn];
   if (blockIdx.x * kClusterThreads >= count) return;
+  if (C.counters[kTall] != 0u) {
+    const uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x;
+    if (i < count) C.nn[i] = paired_place(i, count);
+    return;
+  }
   __shared__ float4 slo[kClusterThreads + 2 * kSearch], shi[kClusterThreads + 2 * kSearch];
   const int base = static_cast<int>(blockIdx.x) * kClusterThreads - kSearch;
   for (int k = threadIdx.x; k < kClusterThreads + 2 * kSearch; k += kClusterThreads) {
@@ -1073,7 +1090,7 @@ __global__ void __launch_bounds__(kClusterThreads) nearest_kernel(Clusters C, co
 // Place i survives unless it merges into a lower place.
 __device__ __forceinline__ bool survives(const Clusters& C, uint32_t i, uint32_t count) {
   if (i >= count) return false;
-  const uint32_t j = C.nn[i];  // none (above i) for a lone cluster
+  const uint32_t j = C.nn[i];  // kNoPlace (above i) for a lone cluster
   return !(j < i && C.nn[j] == i);
 }
 
@@ -1122,14 +1139,15 @@ __global__ void __launch_bounds__(kClusterThreads) merge_kernel(Clusters C, cons
     C.counters[kCount + (turn ^ 1)] = at + (keep ? 1u : 0u);
 }
 
-// The last passes, from at most kFinishThreads clusters to one, in one block: as
-// launches they are small and many (about 30 of a tree's 60 passes). The last
-// cluster's id goes to *root.
+// The last passes, from at most kFinishThreads clusters to one, in one block, by the
+// same rule: as launches they are small and many (about 30 of a tree's 60 passes).
+// The last cluster's id goes to *root.
 constexpr int kFinishThreads = 512;
 __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Clusters C, const uint32_t* ids, uint32_t* root) {
   __shared__ float4 slo[kFinishThreads], shi[kFinishThreads];
   __shared__ uint32_t sid[kFinishThreads], snn[kFinishThreads], warps[kFinishThreads / 32];
   uint32_t count = C.counters[kCount];
+  bool tall = C.counters[kTall] != 0u;
   const uint32_t i = threadIdx.x, lane = i & 31u, warp = i >> 5;
   if (i < count) {
     sid[i] = ids[i];
@@ -1137,11 +1155,13 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Clusters C, cons
     shi[i] = C.hi[ids[i]];
   }
   __syncthreads();
-  for (int pass = 0; count > 1 && pass < kFinishThreads; ++pass) {  // every pass merges a pair: see nearest_place
-    if (i < count) snn[i] = nearest_place(slo, shi, static_cast<int>(i), static_cast<int>(i), static_cast<int>(count));
+  for (int pass = 0; count > 1 && pass < kFinishThreads; ++pass) {  // every pass merges a pair
+    if (i < count)
+      snn[i] = tall ? paired_place(i, count)
+                    : nearest_place(slo, shi, static_cast<int>(i), static_cast<int>(i), static_cast<int>(count));
     __syncthreads();
-    const uint32_t j = i < count ? snn[i] : 0u;
-    const bool mutual = i < count && snn[j] == i, keep = i < count && !(mutual && j < i);
+    const uint32_t j = i < count ? snn[i] : kNoPlace;
+    const bool mutual = j != kNoPlace && snn[j] == i, keep = i < count && !(mutual && j < i);
     float4 lo = {}, hi = {};
     uint32_t id = 0;
     if (keep) {
@@ -1152,7 +1172,7 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Clusters C, cons
     }
     const uint32_t m = __ballot_sync(0xffffffffu, keep);
     if (lane == 0) warps[warp] = __popc(m);
-    __syncthreads();
+    tall = __syncthreads_or(tall || (keep && __float_as_uint(hi.w) >= kMaxHeight)) != 0;
     uint32_t at = __popc(m & ((1u << lane) - 1u)), total = 0;
     for (uint32_t w = 0; w < kFinishThreads / 32; ++w) {
       if (w < warp) at += warps[w];
@@ -1347,7 +1367,7 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
     uint4* node = reinterpret_cast<uint4*>(m + o_node);
     if (e == cudaSuccess) e = cudaMemcpy(d_first, first.data(), (ni + 1) * 4, cudaMemcpyHostToDevice);
     const uint32_t box_init[9] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u};  // centroid bounds; bad flag
-    const uint32_t count_init[kLevelEnd + 2] = {n, n, 0u, 1u, 0u, 0u, 1u};
+    const uint32_t count_init[kLevelEnd + 2] = {n, n, 0u, 1u, 0u, 0u, 0u, 1u};
     if (e == cudaSuccess) e = cudaMemcpy(box, box_init, sizeof(box_init), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(m + o_count, count_init, sizeof(count_init), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(visits, 0, nn * 4 + 4);
@@ -1407,12 +1427,12 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
     uint32_t bad = 0, left = 1;
     if (e == cudaSuccess) e = cudaMemcpy(&bad, box + 8, 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(&left, C.counters + kCount, 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && left != 1) e = cudaErrorUnknown;
+    if (e == cudaSuccess && !bad && (left != 1 || !done)) e = cudaErrorUnknown;  // not for any scene: see kStack
     cudaFree(m);
-    if (e == cudaSuccess && (bad || !done)) {
+    if (e == cudaSuccess && bad) {
       cudaFree(B->block);
       delete B;
-      return bad ? NRC_ERROR_INVALID_ARGUMENT : NRC_ERROR_TOO_LARGE;  // an index past the scene's buffers; see kMaxHeight
+      return NRC_ERROR_INVALID_ARGUMENT;  // an index past the scene's buffers
     }
   }
   if (e != cudaSuccess) {
