@@ -86,3 +86,30 @@ def test_hits_equal_brute_force_past_256_blocks(cuda, oracle):
     from vknrc_gb300 import synthetic as S
 
     _compare(oracle, _triangles("random", 70000, S.rng_for(70)), 32, 20)
+
+
+def test_build_time_is_bounded(cuda):
+    """Triangles whose boxes grow along the order take a bounded number of passes: one
+    merge a pass is some hundred times as long as an ordinary scene's build."""
+    import time
+
+    import torch
+
+    from vknrc_gb300 import nrc, synthetic as S
+
+    n, best = 60000, []
+    for kind in ("random", "nested along z"):
+        sc = S.scene(S.rng_for(3), vertices=300, primitives=100, instances=1)
+        for k in ("texcoord_indices", "material_ids"):
+            sc[k] = np.resize(sc[k], (n,) + sc[k].shape[1:])
+        sc["vertices"] = _triangles(kind, n, S.rng_for(n)).reshape(-1, 3).astype(np.float32)
+        sc["vertex_indices"] = np.arange(3 * n, dtype=np.uint32).reshape(n, 3)
+        sc["instance_ranges"] = np.array([[0, n]], np.uint32)
+        ds, times = nrc.DeviceScene(sc), []
+        for _ in range(4):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            nrc.Bvh(ds).close()
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+    assert best[1] < 15 * best[0], best
