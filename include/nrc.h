@@ -683,7 +683,7 @@ typedef struct nrc_bvh nrc_bvh;
 /* Builds a BVH over every instance's transformed triangles on the current
  * device (triangles in Morton order, clustered bottom-up by box area, the binary
  * tree collapsed to four-wide nodes; `nodes` of nrc_bvh_info counts the binary
- * ones). Coordinates up to 1e15. d_ranges: instance_count entries in device memory. Synchronous. */
+ * ones). d_ranges: instance_count entries in device memory. Synchronous. */
 NRC_API int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nrc_bvh** out);
 NRC_API int nrc_bvh_destroy(nrc_bvh* bvh);
 NRC_API int nrc_bvh_info(const nrc_bvh* bvh, uint32_t* triangles, uint32_t* nodes);

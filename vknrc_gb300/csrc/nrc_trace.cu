@@ -420,6 +420,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
+// A ray's offset in the slab test of an axis, coordinate p being met at p * i + o. Where
+// it overflows it is NaN, which max3 and min3 pass over: the axis then excludes no box.
+__device__ __forceinline__ float slab_offset(float origin, float i) {
+  const float o = -origin * i;
+  return fabsf(o) < __int_as_float(0x7F800000) ? o : __int_as_float(0x7FC00000);
+}
 __device__ __forceinline__ float min3(float a, float b, float c) {
   float r;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -447,10 +453,12 @@ __device__ __noinline__ int trace_closest(const TriView B, Ray r, float tmin, fl
   const float ix = fabsf(r.d.x) > 1e-20f ? 1.0f / r.d.x : copysignf(1e20f, r.d.x);
   const float iy = fabsf(r.d.y) > 1e-20f ? 1.0f / r.d.y : copysignf(1e20f, r.d.y);
   const float iz = fabsf(r.d.z) > 1e-20f ? 1.0f / r.d.z : copysignf(1e20f, r.d.z);
-  const float ox = -r.o.x * ix, oy = -r.o.y * iy, oz = -r.o.z * iz;  // coordinate p is met at p * i + o
+  const float ox = slab_offset(r.o.x, ix), oy = slab_offset(r.o.y, iy), oz = slab_offset(r.o.z, iz);
   const int sx = ix >= 0.0f ? 0 : 1, sy = iy >= 0.0f ? 0 : 1, sz = iz >= 0.0f ? 0 : 1;  // which of the planes is near
-  // A ray with a NaN meets nothing (every comparison of the triangle test fails).
+  // A ray with a NaN or an infinity meets nothing (every comparison of the triangle test fails).
   const float sum = (r.o.x + r.o.y + r.o.z) + (r.d.x + r.d.y + r.d.z);
+  const float most = fmaxf(max3(fabsf(r.o.x), fabsf(r.o.y), fabsf(r.o.z)), max3(fabsf(r.d.x), fabsf(r.d.y), fabsf(r.d.z)));
+  const bool finite = sum == sum && most < __int_as_float(0x7F800000);
   constexpr uint32_t kRoot = (1u << 24) | 1u;
   int best = -1;
   float bt = tmax;
@@ -459,7 +467,7 @@ __device__ __noinline__ int trace_closest(const TriView B, Ray r, float tmin, fl
   // and the slots holding nodes (bits 0..3). The root is slot 0 of its own group.
   uint2 stack[kStack];
   int sp = 0;
-  uint32_t base = 0, group = sum == sum ? kRoot : 0u;
+  uint32_t base = 0, group = finite ? kRoot : 0u;
   uint32_t tri0 = 0, tset = 0, tri1 = 0, tset1 = 0;  // pending triangles of two nodes: first, present << 12 | hit
   bool strict = false;  // test the guard box of every hit, not only of the closest
   const uint32_t lanes = __activemask();
@@ -875,6 +883,7 @@ __global__ void morton_kernel(const float* cent, uint32_t n, const uint32_t* box
 constexpr int kSearch = 16, kClusterThreads = 256, kBatch = 8;
 constexpr uint32_t kLeafTris = 3;
 constexpr uint32_t kNoPlace = 0xFFFFFFFFu;
+constexpr float kFarthest = 1e15f;
 
 struct Clusters {
   float4 *lo, *hi;  // box per id; lo.w triangles below, hi.w height (as bits)
@@ -901,7 +910,8 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 // lengths, 0.4 to 10%, whatever the margin between 1e-5 and 1/64 of the length. Wider
 // boxes cost the traversal: 1/64 and 1e-4 of the coordinates 1,709 us for a rendered
 // 1080p frame, 1/256 and 1e-5 1,629, 1/1024 1,581. The triangle's cluster starts from
-// that box, kept within +-1e15, so that no term of the traversal's slab test overflows.
+// that box, kept within +-kFarthest: half_area stays finite, and so do the traversal's
+// slab terms, at most 1e20 times a coordinate (see widen for what lies beyond).
 __global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const float4* tri, float4* guard, uint32_t* ids) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= C.n) return;
@@ -920,8 +930,8 @@ __global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const flo
   guard[size_t(t) * 2 + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
   for (int k = 0; k < 3; ++k) {
     if (!(lo[k] <= hi[k])) lo[k] = hi[k] = 0.0f;  // no finite vertex: the triangle is never hit
-    lo[k] = fminf(fmaxf(lo[k], -1e15f), 1e15f);
-    hi[k] = fminf(fmaxf(hi[k], -1e15f), 1e15f);
+    lo[k] = fminf(fmaxf(lo[k], -kFarthest), kFarthest);
+    hi[k] = fminf(fmaxf(hi[k], -kFarthest), kFarthest);
   }
   C.lo[i] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(1u));
   C.hi[i] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(0u));
@@ -1118,7 +1128,8 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Clusters C, cons
 // until it has four (clusters of more than three triangles before smaller
 // ones); what is left of up to three triangles becomes a leaf. The next level's
 // nodes are appended to cluster_of. Boxes are widened by 1e-6 of their
-// coordinates: the traversal's p * i + o rounds by less.
+// coordinates: the traversal's p * i + o rounds by less. A box that reaches
+// +-kFarthest has no plane on that side.
 __device__ __forceinline__ void widen(const Clusters& C, uint32_t* cluster_of, uint32_t w, const uint32_t* order,
                                       const float4* tri, WideNode* wide, float4* leaf) {
   uint32_t c[4] = {cluster_of[w], 0u, 0u, 0u};
@@ -1167,8 +1178,8 @@ __device__ __forceinline__ void widen(const Clusters& C, uint32_t* cluster_of, u
     const float l3[3] = {lo.x, lo.y, lo.z}, h3[3] = {hi.x, hi.y, hi.z};
     for (int a = 0; a < 3; ++a) {
       const float pad = fmaxf(fabsf(l3[a]), fabsf(h3[a])) * 1e-6f;
-      plane[8 * a + s] = l3[a] - pad;
-      plane[8 * a + 4 + s] = h3[a] + pad;
+      plane[8 * a + s] = l3[a] > -kFarthest ? l3[a] - pad : -inf;
+      plane[8 * a + 4 + s] = h3[a] < kFarthest ? h3[a] + pad : inf;
     }
     const uint32_t tris = __float_as_uint(lo.w);
     if (tris > kLeafTris) {
