@@ -73,7 +73,7 @@ def _compare(oracle, tri, w, h):
     bvh.close()
 
 
-@pytest.mark.parametrize("kind,n", [("random", k) for k in (511, 512, 513, 769, 1024, 3000)] +
+@pytest.mark.parametrize("kind,n", [("random", k) for k in (511, 512, 513, 769, 1023, 1024, 1025, 3000, 8192, 8193)] +
                          [("identical", 513), ("identical", 3000), ("wall", 2000), ("never hit", 2000), ("gaps", 4000),
                           ("nested", 8000), ("nested along z", 4000)])
 def test_hits_equal_brute_force(cuda, oracle, kind, n):

@@ -373,8 +373,8 @@ struct TriView {
 };
 
 // A traversal stacks at most one entry per level of the wide tree, which has at
-// most as many as the binary tree under it is high: kMaxHeight, after which every
-// clustering pass halves what is left of fewer than 2^30 clusters.
+// most as many as the binary tree under it is high: kMaxHeight, and the passes that
+// halve what is left of fewer than 2^30 clusters, at most 30 (see cluster_kernel).
 constexpr uint32_t kMaxHeight = 48;
 constexpr int kStack = kMaxHeight + 32;
 
@@ -867,20 +867,24 @@ __global__ void morton_kernel(const float* cent, uint32_t n, const uint32_t* box
 // Parallel locally-ordered clustering (Meister and Bittner 2018) over the
 // triangles in Morton order: each cluster looks kSearch places to either side for
 // the one whose union with it has the least area; pairs that choose each other
-// merge; the survivors keep their order. Unlike the radix tree, a triangle much
+// merge; the survivors keep their order. Unlike a radix tree's, a triangle much
 // larger than its neighbours (a wall beside a tessellated floor) joins late,
 // near the root, instead of stretching the boxes of everything above a small one.
-// Ids: a triangle in Morton order at [0, n), merged clusters from n on.
-// Two rules keep that bounded for every scene. Once a cluster is kMaxHeight high,
-// all later passes pair the clusters by place (even with odd): each halves them, so
-// the tree gets at most 30 higher. And when a batch of kBatch passes leaves more than
-// half of the clusters, the next pass pairs by place, so n triangles take about
-// 16 log2(n) passes at most: boxes that grow along the order choose their lower
-// neighbour one and all, and only one pair of such a run is mutual. (4,000 triangles
-// nested in one another: 57 passes and 57 high, by the search alone 3,919 and 129;
-// along an axis, whose tree is lower, 120 passes instead of 3,501. 20,000 small
-// random triangles: 39 passes, 19 high either way.)
-constexpr int kSearch = 16, kClusterThreads = 256, kBatch = 8;
+// It runs in stages, each one launch: a block takes kChunk places in a row through
+// the passes (three or four) that leave kKeep clusters, the next stage's blocks take
+// the survivors of kFan blocks each, and the last stage's one block goes on to a single
+// cluster. No pair forms across a chunk's edge in a stage, which hardly matters: over 22
+// scenes the traced frames take 0.99 of the time with passes over all places, a single
+// one 0.9 to 1.1 either way (where a room's few large triangles land), and chunks of 256
+// to 1,024 places with a half to a sixteenth kept 0.99 to 1.03. Nothing is read back.
+// Passes over all places, three launches each and a read-back every eight, took the
+// build of 7,950 triangles 0.99 ms and of 522,254 1.77; these stages, with the widening
+// below, 0.48 and 0.82.
+// Ids: a triangle in Morton order at [0, n), merged clusters from n on. A cluster is
+// represented by its first triangle's place in that order; merging i with a higher
+// place j gives up j's, so the merged cluster's id is n + that one.
+constexpr uint32_t kSearch = 16, kBatch = 8;
+constexpr uint32_t kChunk = 512, kKeep = 256, kFan = kChunk / kKeep;
 constexpr uint32_t kLeafTris = 3;
 constexpr uint32_t kNoPlace = 0xFFFFFFFFu;
 constexpr float kFarthest = 1e15f;
@@ -888,16 +892,12 @@ constexpr float kFarthest = 1e15f;
 struct Clusters {
   float4 *lo, *hi;  // box per id; lo.w triangles below, hi.w height (as bits)
   uint2* child;     // of id n + i
-  uint32_t* nn;     // chosen neighbour (place) of each place
-  uint32_t* kept;   // survivors per block, then per kClusterThreads blocks (from kept + kept_blocks)
-  uint32_t kept_blocks;
-  uint32_t* counters;  // see kNextId ..
   uint32_t n;
 };
-// Counters: the next cluster id; the clusters before and after a pass (in turn);
-// wide nodes and leaf triangles so far; whether a cluster is kMaxHeight high; the
-// wide nodes up to each level (from 0).
-constexpr int kNextId = 0, kCount = 1, kWide = 3, kLeafs = 4, kTall = 5, kLevelEnd = 6, kCounters = kLevelEnd + kStack + 6;
+// The build's counters: a vertex index was out of range; wide nodes and leaf
+// triangles so far; clusters left (one); the widening's nodes for its second launch
+// (first, count); the bounds of the centroids.
+constexpr int kBad = 0, kWide = 1, kLeafs = 2, kLeft = 3, kFrontier = 4, kBox = 6, kCounters = 12;
 
 __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
   const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
@@ -912,10 +912,7 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 // 1080p frame, 1/256 and 1e-5 1,629, 1/1024 1,581. The triangle's cluster starts from
 // that box, kept within +-kFarthest: half_area stays finite, and so do the traversal's
 // slab terms, at most 1e20 times a coordinate (see widen for what lies beyond).
-__global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const float4* tri, float4* guard, uint32_t* ids) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C.n) return;
-  const uint32_t t = order[i];
+__device__ __forceinline__ void triangle_boxes(const float4* tri, uint32_t t, float4* guard, float4& clo, float4& chi) {
   const float4 v0 = tri[size_t(t) * 3], v1 = tri[size_t(t) * 3 + 1], v2 = tri[size_t(t) * 3 + 2];
   float lo[3] = {fminf(fminf(v0.x, v1.x), v2.x), fminf(fminf(v0.y, v1.y), v2.y), fminf(fminf(v0.z, v1.z), v2.z)};
   float hi[3] = {fmaxf(fmaxf(v0.x, v1.x), v2.x), fmaxf(fmaxf(v0.y, v1.y), v2.y), fmaxf(fmaxf(v0.z, v1.z), v2.z)};
@@ -933,287 +930,338 @@ __global__ void cluster_init_kernel(Clusters C, const uint32_t* order, const flo
     lo[k] = fminf(fmaxf(lo[k], -kFarthest), kFarthest);
     hi[k] = fminf(fmaxf(hi[k], -kFarthest), kFarthest);
   }
-  C.lo[i] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(1u));
-  C.hi[i] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(0u));
-  ids[i] = i;
+  clo = make_float4(lo[0], lo[1], lo[2], __uint_as_float(1u));
+  chi = make_float4(hi[0], hi[1], hi[2], __uint_as_float(0u));
 }
 
-// The place that place i of `count` pairs with by place alone.
-__device__ __forceinline__ uint32_t paired_place(uint32_t i, uint32_t count) {
-  return (i ^ 1u) < count ? i ^ 1u : kNoPlace;
-}
-
-// The place that place i of `count` chooses; lo and hi hold the boxes, place i's at
-// index `at`. Equal areas choose the nearer place, then the pair that starts at an
-// even place, then the lower place, so that runs of equal boxes pair up and some
-// pair always chooses each other: of the pairs with the least area, distance and
-// parity, the lowest does.
-__device__ __forceinline__ uint32_t nearest_place(const float4* lo, const float4* hi, int at, int i, int count) {
-  const float4 l = lo[at], h = hi[at];
-  float best_d = 0.0f;
-  uint32_t best_k = 0, best_j = kNoPlace;
-  for (int o = -kSearch; o <= kSearch; ++o) {
-    const int j = i + o;
-    if (o == 0 || j < 0 || j >= count) continue;
-    const float4 a = lo[at + o], b = hi[at + o];
-    const float d = half_area(make_float4(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z), 0.0f),
-                              make_float4(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z), 0.0f));
-    const uint32_t key = 2u * static_cast<uint32_t>(abs(o)) + (static_cast<uint32_t>(min(i, j)) & 1u);
-    if (best_j == kNoPlace || d < best_d || (d == best_d && key < best_k)) {
-      best_d = d;
-      best_k = key;
-      best_j = static_cast<uint32_t>(j);
+// A stage of the clustering: `in` holds the survivors (id, representative) of the
+// previous stage's `chunks` blocks, kKeep places each, in_count[b] of them used; the
+// first stage (in null) takes the triangles and makes their boxes. Leaves at most
+// `keep` clusters of the block in out, their number in out_count.
+// Equal areas choose the nearer place, then the pair that starts at an even place,
+// then the lower place, so that runs of equal boxes pair up and some pair always
+// chooses each other: of the pairs with the least area, distance and parity, the
+// lowest does. Two rules keep height and passes bounded for every scene. Once a cluster
+// is kMaxHeight high, all later passes of its block pair the clusters by place (even
+// with odd), which halves them: one such pass in each of up to 21 stages and nine in the
+// last. And when a batch of kBatch passes leaves more than half of the clusters, the
+// next pass pairs by place: boxes that grow along the order choose their lower
+// neighbour one and all, and only one pair of such a run is mutual. (4,000 triangles
+// nested in one another: 56 high after 56 passes, by the search alone 129 and 3,919.)
+// A full pass is bound by the minima and maxima of the areas, each pair's computed once
+// and read by both places (twice, for either place: 7,700 cycles a pass, and 1.04 ms for
+// the build of 522,254 triangles); with few clusters left, several lanes share one's
+// pairs, and a pass is its barriers and shared-memory latency.
+__global__ void __launch_bounds__(kChunk) cluster_kernel(Clusters C, const uint32_t* order, const float4* tri, float4* guard,
+                                                         const uint2* in, const uint32_t* in_count, uint32_t chunks,
+                                                         uint32_t keep, uint2* out, uint32_t* out_count) {
+  extern __shared__ float4 cluster_smem[];
+  float4 *const slo = cluster_smem, *const shi = slo + kChunk;
+  float* const pair_area = reinterpret_cast<float*>(shi + kChunk);  // [kSearch][kChunk]
+  __shared__ uint32_t sid[kChunk], srep[kChunk], snn[kChunk], warps[kChunk / 32];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  uint32_t count = 0;
+  bool tall = false;
+  if (in == nullptr) {
+    const uint32_t first = blockIdx.x * kChunk;
+    count = min(C.n - first, kChunk);
+    if (t < count) {
+      float4 lo, hi;
+      triangle_boxes(tri, order[first + t], guard, lo, hi);
+      C.lo[first + t] = slo[t] = lo;
+      C.hi[first + t] = shi[t] = hi;
+      sid[t] = srep[t] = first + t;
+    }
+  } else {
+    const uint32_t first = blockIdx.x * kFan, mine = first + t / kKeep;
+    uint32_t at = t % kKeep, n = 0;
+    for (uint32_t b = first; b < min(first + kFan, chunks); ++b) {
+      const uint32_t c = in_count[b];
+      if (b < mine) at += c;
+      if (b == mine) n = c;
+      count += c;
+    }
+    if (t % kKeep < n) {
+      const uint2 v = in[size_t(mine) * kKeep + t % kKeep];
+      sid[at] = v.x;
+      srep[at] = v.y;
+      slo[at] = C.lo[v.x];
+      const float4 hi = C.hi[v.x];
+      shi[at] = hi;
+      tall = __float_as_uint(hi.w) >= kMaxHeight;
     }
   }
-  return best_j;
-}
-
-// Merges clusters `id` and `other` (their boxes given): the new id, its box in lo, hi.
-// The first to be kMaxHeight high sets counters[kTall], which the next pass reads.
-__device__ __forceinline__ uint32_t merge_clusters(const Clusters& C, uint32_t id, uint32_t other, float4& lo, float4& hi,
-                                                   float4 olo, float4 ohi) {
-  const uint32_t merged = atomicAdd(&C.counters[kNextId], 1u);
-  lo = make_float4(fminf(lo.x, olo.x), fminf(lo.y, olo.y), fminf(lo.z, olo.z),
-                   __uint_as_float(__float_as_uint(lo.w) + __float_as_uint(olo.w)));
-  hi = make_float4(fmaxf(hi.x, ohi.x), fmaxf(hi.y, ohi.y), fmaxf(hi.z, ohi.z),
-                   __uint_as_float(max(__float_as_uint(hi.w), __float_as_uint(ohi.w)) + 1u));
-  if (__float_as_uint(hi.w) >= kMaxHeight) C.counters[kTall] = 1u;
-  C.lo[merged] = lo;
-  C.hi[merged] = hi;
-  C.child[merged - C.n] = make_uint2(id, other);
-  return merged;
-}
-
-// The passes run in batches, grids sized by the count before the batch: the
-// count of a pass is in counters[kCount + turn].
-__global__ void __launch_bounds__(kClusterThreads) nearest_kernel(Clusters C, const uint32_t* ids, int turn, bool by_place) {
-  const uint32_t count = C.counters[kCount + turn];
-  if (blockIdx.x * kClusterThreads >= count) return;
-  if (threadIdx.x == 0 && blockIdx.x % kClusterThreads == 0) C.kept[C.kept_blocks + blockIdx.x / kClusterThreads] = 0u;
-  if (by_place || C.counters[kTall] != 0u) {
-    const uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x;
-    if (i < count) C.nn[i] = paired_place(i, count);
-    return;
-  }
-  __shared__ float4 slo[kClusterThreads + 2 * kSearch], shi[kClusterThreads + 2 * kSearch];
-  const int base = static_cast<int>(blockIdx.x) * kClusterThreads - kSearch;
-  for (int k = threadIdx.x; k < kClusterThreads + 2 * kSearch; k += kClusterThreads) {
-    const int j = base + k;
-    if (j >= 0 && j < static_cast<int>(count)) {
-      slo[k] = C.lo[ids[j]];
-      shi[k] = C.hi[ids[j]];
+  tall = __syncthreads_or(tall) != 0;
+  uint32_t batch_count = count;
+  bool by_place = false;
+  for (uint32_t pass = 1; count > keep && pass < kChunk; ++pass) {  // every pass merges a pair
+    if (tall || by_place) {
+      if (t < count) snn[t] = (t ^ 1u) < count ? t ^ 1u : kNoPlace;
+    } else {
+      const uint32_t share = min(__clz(count - 1u) - __clz(kChunk - 1u), 4), lanes = 1u << share;  // lanes a place: count << share <= kChunk
+      const uint32_t i = t >> share, sub = t & (lanes - 1u);
+      const float inf = __int_as_float(0x7F800000);
+      if (i < count) {
+        const float4 l = slo[i], h = shi[i];
+#pragma unroll 4
+        for (uint32_t o = sub; o < kSearch; o += lanes) {  // the pair of places i and i + o + 1
+          float d = inf;
+          if (i + o + 1 < count) {
+            const float4 a = slo[i + o + 1], b = shi[i + o + 1];
+            d = half_area(make_float4(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z), 0.0f),
+                          make_float4(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z), 0.0f));
+          }
+          pair_area[o * kChunk + i] = d;
+        }
+      }
+      __syncthreads();
+      float best_d = inf;
+      int best_o = 0;
+      if (i < count) {
+#pragma unroll 4
+        for (uint32_t o = sub; o < kSearch; o += lanes) {
+          const float above = pair_area[o * kChunk + i], below = i > o ? pair_area[o * kChunk + i - o - 1] : inf;
+          const bool up = above < below || (above == below && ((i | o) & 1u) == 0u);  // an odd distance from an even place
+          const float d = up ? above : below;
+          if (d < best_d) {
+            best_d = d;
+            best_o = up ? static_cast<int>(o) + 1 : -static_cast<int>(o) - 1;
+          }
+        }
+      }
+      for (uint32_t off = 1; off < lanes; off <<= 1) {
+        const float d = __shfl_xor_sync(0xffffffffu, best_d, off);
+        const int o = __shfl_xor_sync(0xffffffffu, best_o, off);
+        if (d < best_d || (d == best_d && abs(o) < abs(best_o))) {
+          best_d = d;
+          best_o = o;
+        }
+      }
+      if (i < count && sub == 0u) snn[i] = i + best_o;
     }
-  }
-  __syncthreads();
-  const int at = static_cast<int>(threadIdx.x) + kSearch, i = base + at;
-  if (i < static_cast<int>(count)) C.nn[i] = nearest_place(slo, shi, at, i, static_cast<int>(count));
-}
-
-// Place i survives unless it merges into a lower place.
-__device__ __forceinline__ bool survives(const Clusters& C, uint32_t i, uint32_t count) {
-  if (i >= count) return false;
-  const uint32_t j = C.nn[i];  // kNoPlace (above i) for a lone cluster
-  return !(j < i && C.nn[j] == i);
-}
-
-__global__ void __launch_bounds__(kClusterThreads) kept_kernel(Clusters C, int turn) {
-  const uint32_t count = C.counters[kCount + turn];
-  if (blockIdx.x * kClusterThreads >= count) return;
-  const uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x;
-  const int k = __syncthreads_count(survives(C, i, count) ? 1 : 0);
-  if (threadIdx.x == 0) {
-    C.kept[blockIdx.x] = static_cast<uint32_t>(k);
-    atomicAdd(&C.kept[C.kept_blocks + blockIdx.x / kClusterThreads], static_cast<uint32_t>(k));
-  }
-}
-
-__global__ void __launch_bounds__(kClusterThreads) merge_kernel(Clusters C, const uint32_t* ids, uint32_t* out,
-                                                                int turn) {
-  const uint32_t count = C.counters[kCount + turn];
-  if (blockIdx.x * kClusterThreads >= count) return;
-  __shared__ uint32_t before[kClusterThreads / 32], warps[kClusterThreads / 32];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  // survivors of the blocks before this one: whole groups of blocks, then the blocks of its own
-  const uint32_t group = blockIdx.x / kClusterThreads, before_it = group * kClusterThreads + threadIdx.x;
-  uint32_t sum = before_it < blockIdx.x ? C.kept[before_it] : 0u;
-  for (uint32_t g = threadIdx.x; g < group; g += kClusterThreads) sum += C.kept[C.kept_blocks + g];
-  sum = __reduce_add_sync(0xffffffffu, sum);
-  const uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x;
-  const bool keep = survives(C, i, count);
-  const uint32_t m = __ballot_sync(0xffffffffu, keep);
-  if (lane == 0) {
-    before[warp] = sum;
-    warps[warp] = __popc(m);
-  }
-  __syncthreads();
-  uint32_t at = __popc(m & ((1u << lane) - 1u));
-  for (uint32_t w = 0; w < kClusterThreads / 32; ++w) {
-    at += before[w];
-    if (w < warp) at += warps[w];
-  }
-  if (keep) {
-    uint32_t id = ids[i];
-    const uint32_t j = C.nn[i];
-    if (j > i && j < count && C.nn[j] == i) {  // merges with a higher place
-      const uint32_t other = ids[j];
-      float4 lo = C.lo[id], hi = C.hi[id];
-      id = merge_clusters(C, id, other, lo, hi, C.lo[other], C.hi[other]);
-    }
-    out[at] = id;
-  }
-  if (blockIdx.x == (count - 1) / kClusterThreads && threadIdx.x == kClusterThreads - 1)
-    C.counters[kCount + (turn ^ 1)] = at + (keep ? 1u : 0u);
-}
-
-// The last passes, from at most kFinishThreads clusters to one, in one block, by the
-// same rules: as launches they are small and many (about 30 of a tree's 60 passes).
-// The last cluster's id goes to *root.
-constexpr int kFinishThreads = 512;
-__global__ void __launch_bounds__(kFinishThreads) finish_kernel(Clusters C, const uint32_t* ids, uint32_t* root) {
-  __shared__ float4 slo[kFinishThreads], shi[kFinishThreads];
-  __shared__ uint32_t sid[kFinishThreads], snn[kFinishThreads], warps[kFinishThreads / 32];
-  uint32_t count = C.counters[kCount], batch_count = count;
-  bool tall = C.counters[kTall] != 0u, by_place = false;
-  const uint32_t i = threadIdx.x, lane = i & 31u, warp = i >> 5;
-  if (i < count) {
-    sid[i] = ids[i];
-    slo[i] = C.lo[ids[i]];
-    shi[i] = C.hi[ids[i]];
-  }
-  __syncthreads();
-  for (int pass = 0; count > 1 && pass < kFinishThreads; ++pass) {  // every pass merges a pair
-    if (i < count)
-      snn[i] = tall || by_place ? paired_place(i, count)
-                                : nearest_place(slo, shi, static_cast<int>(i), static_cast<int>(i), static_cast<int>(count));
     __syncthreads();
-    const uint32_t j = i < count ? snn[i] : kNoPlace;
-    const bool mutual = j != kNoPlace && snn[j] == i, keep = i < count && !(mutual && j < i);
+    const uint32_t j = t < count ? snn[t] : kNoPlace;
+    const bool mutual = j != kNoPlace && snn[j] == t, kept = t < count && !(mutual && j < t);
     float4 lo = {}, hi = {};
-    uint32_t id = 0;
-    if (keep) {
-      id = sid[i];
-      lo = slo[i];
-      hi = shi[i];
-      if (mutual) id = merge_clusters(C, id, sid[j], lo, hi, slo[j], shi[j]);
+    uint32_t id = 0, rep = 0;
+    if (kept) {
+      id = sid[t];
+      rep = srep[t];
+      lo = slo[t];
+      hi = shi[t];
+      if (mutual) {
+        const float4 a = slo[j], b = shi[j];
+        const uint32_t merged = srep[j];
+        C.child[merged] = make_uint2(id, sid[j]);
+        id = C.n + merged;
+        lo = make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z),
+                         __uint_as_float(__float_as_uint(lo.w) + __float_as_uint(a.w)));
+        hi = make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z),
+                         __uint_as_float(max(__float_as_uint(hi.w), __float_as_uint(b.w)) + 1u));
+        C.lo[id] = lo;
+        C.hi[id] = hi;
+      }
     }
-    const uint32_t m = __ballot_sync(0xffffffffu, keep);
+    const uint32_t m = __ballot_sync(0xffffffffu, kept);
     if (lane == 0) warps[warp] = __popc(m);
-    tall = __syncthreads_or(tall || (keep && __float_as_uint(hi.w) >= kMaxHeight)) != 0;
-    uint32_t at = __popc(m & ((1u << lane) - 1u)), total = 0;
-    for (uint32_t w = 0; w < kFinishThreads / 32; ++w) {
-      if (w < warp) at += warps[w];
-      total += warps[w];
-    }
-    if (keep) {
+    tall = __syncthreads_or(tall || (kept && __float_as_uint(hi.w) >= kMaxHeight)) != 0;
+    const uint32_t of_warp = lane < kChunk / 32 ? warps[lane] : 0u;
+    const uint32_t at = __popc(m & ((1u << lane) - 1u)) + __reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0u);
+    const uint32_t total = __reduce_add_sync(0xffffffffu, of_warp);
+    if (kept) {
       sid[at] = id;
+      srep[at] = rep;
       slo[at] = lo;
       shi[at] = hi;
     }
     count = total;
     by_place = false;
-    if (pass % kBatch == kBatch - 1) {
+    if (pass % kBatch == 0) {
       by_place = count > batch_count / 2;
       batch_count = count;
     }
     __syncthreads();
   }
-  if (i == 0) {
-    *root = sid[0];
-    C.counters[kCount] = count;
-  }
+  if (t < min(count, keep)) out[size_t(blockIdx.x) * kKeep + t] = make_uint2(sid[t], srep[t]);
+  if (t == 0) out_count[blockIdx.x] = count;
 }
 
-// One level of the wide tree: its nodes w, each over the binary cluster
-// cluster_of[w]. A node starts from its cluster and opens the largest
-// until it has four (clusters of more than three triangles before smaller
-// ones); what is left of up to three triangles becomes a leaf. The next level's
-// nodes are appended to cluster_of. Boxes are widened by 1e-6 of their
-// coordinates: the traversal's p * i + o rounds by less. A box that reaches
-// +-kFarthest has no plane on that side.
-__device__ __forceinline__ void widen(const Clusters& C, uint32_t* cluster_of, uint32_t w, const uint32_t* order,
-                                      const float4* tri, WideNode* wide, float4* leaf) {
-  uint32_t c[4] = {cluster_of[w], 0u, 0u, 0u};
-  int k = 1;
-  while (k < 4) {
-    int pick = -1;
-    bool pick_large = false;
-    float pick_area = 0.0f;
-    for (int x = 0; x < k; ++x) {
-      const float4 lo = C.lo[c[x]];
-      const uint32_t tris = __float_as_uint(lo.w);
-      if (tris < 2) continue;
-      const bool large = tris > kLeafTris;
-      const float area = half_area(lo, C.hi[c[x]]);
-      if (pick < 0 || (large && !pick_large) || (large == pick_large && area > pick_area)) {
-        pick = x;
-        pick_large = large;
-        pick_area = area;
+// The wide tree's nodes first .. first + count (at most T), each over the binary
+// cluster cluster_of[w]. A node starts from its cluster and opens the largest until it
+// has four (clusters of more than three triangles before smaller ones); what is left
+// of up to three triangles becomes a leaf, whose triangles (in Morton order) go to
+// leaf_of. The nodes' children are appended to the tree as one range, which is
+// returned. Boxes are widened by 1e-6 of their coordinates: the traversal's p * i + o
+// rounds by less. A box that reaches +-kFarthest has no plane on that side.
+template <uint32_t T>
+__device__ __forceinline__ uint2 widen(const Clusters& C, uint32_t* cluster_of, uint32_t* counters, uint32_t first,
+                                       uint32_t count, WideNode* wide, uint32_t* leaf_of) {
+  __shared__ uint32_t sums[T / 32], base[2];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  const bool in = t < count;
+  float4 lo[4], hi[4];
+  uint32_t c[4] = {0u, 0u, 0u, 0u};
+  int k = 0;
+  if (in) {
+    c[0] = cluster_of[first + t];
+    lo[0] = C.lo[c[0]];
+    hi[0] = C.hi[c[0]];
+    k = 1;
+#pragma unroll
+    for (int s = 1; s < 4; ++s) {
+      int pick = -1;
+      bool pick_large = false;
+      float pick_area = 0.0f;
+      uint32_t id = 0;
+#pragma unroll
+      for (int x = 0; x < s; ++x) {
+        const uint32_t tris = __float_as_uint(lo[x].w);
+        const bool large = tris > kLeafTris;
+        const float area = half_area(lo[x], hi[x]);
+        if (tris >= 2 && (pick < 0 || (large && !pick_large) || (large == pick_large && area > pick_area))) {
+          pick = x;
+          pick_large = large;
+          pick_area = area;
+          id = c[x];
+        }
       }
+      if (pick < 0) break;
+      const uint2 ch = C.child[id - C.n];
+      const float4 al = C.lo[ch.x], ah = C.hi[ch.x];
+#pragma unroll
+      for (int x = 0; x < s; ++x)
+        if (x == pick) {
+          c[x] = ch.x;
+          lo[x] = al;
+          hi[x] = ah;
+        }
+      c[s] = ch.y;
+      lo[s] = C.lo[ch.y];
+      hi[s] = C.hi[ch.y];
+      k = s + 1;
     }
-    if (pick < 0) break;
-    const uint2 ch = C.child[c[pick] - C.n];
-    c[pick] = ch.x;
-    c[k++] = ch.y;
   }
-  uint32_t nodes = 0, leaf_tris = 0;
-  for (int s = 0; s < k; ++s) {
-    const uint32_t tris = __float_as_uint(C.lo[c[s]].w);
-    if (tris > kLeafTris) ++nodes; else leaf_tris += tris;
+  uint32_t nodes = 0, tris = 0;
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+    if (s < k) {
+      const uint32_t below = __float_as_uint(lo[s].w);
+      if (below > kLeafTris) ++nodes; else tris += below;
+    }
+  // the block's ranges of nodes and leaf triangles, this thread's places in them (counts of both in one word)
+  const uint32_t own = nodes | tris << 16;
+  uint32_t upto = own;
+#pragma unroll
+  for (uint32_t off = 1; off < 32; off <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
+    if (lane >= off) upto += v;
   }
-  WideNode N = {};
-  N.node0 = atomicAdd(&C.counters[kWide], nodes);
-  N.tri0 = atomicAdd(&C.counters[kLeafs], leaf_tris);
-  uint32_t node_at = N.node0, tri_at = N.tri0;
-  float* plane = reinterpret_cast<float*>(N.plane);  // [6][4]
-  const float inf = __int_as_float(0x7F800000);
-  for (int s = 0; s < 4; ++s) {
-    if (s >= k) {
-      for (int a = 0; a < 3; ++a) {
-        plane[8 * a + s] = inf;
-        plane[8 * a + 4 + s] = -inf;
-      }
-      continue;
-    }
-    const float4 lo = C.lo[c[s]], hi = C.hi[c[s]];
-    const float l3[3] = {lo.x, lo.y, lo.z}, h3[3] = {hi.x, hi.y, hi.z};
-    for (int a = 0; a < 3; ++a) {
-      const float pad = fmaxf(fabsf(l3[a]), fabsf(h3[a])) * 1e-6f;
-      plane[8 * a + s] = l3[a] > -kFarthest ? l3[a] - pad : -inf;
-      plane[8 * a + 4 + s] = h3[a] < kFarthest ? h3[a] + pad : inf;
-    }
-    const uint32_t tris = __float_as_uint(lo.w);
-    if (tris > kLeafTris) {
-      N.contents |= 1u << (24 + s);
-      cluster_of[node_at++] = c[s];
-      continue;
-    }
-    N.contents |= ((1u << tris) - 1u) << (3 * s);
-    // the cluster's triangles (at most three): left child first
-    uint32_t todo[3] = {c[s], 0u, 0u};
-    for (int sp = 1; sp > 0;) {
-      const uint32_t x = todo[--sp];
-      if (x >= C.n) {
-        const uint2 ch = C.child[x - C.n];
-        todo[sp++] = ch.y;
-        todo[sp++] = ch.x;
+  if (lane == 31) sums[warp] = upto;
+  __syncthreads();
+  uint32_t before = upto - own, total = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < T / 32; ++w) {
+    if (w < warp) before += sums[w];
+    total += sums[w];
+  }
+  if (t < 2) base[t] = atomicAdd(&counters[kWide + t], t == 0 ? total & 0xFFFFu : total >> 16);
+  __syncthreads();
+  const uint2 next = make_uint2(base[0], total & 0xFFFFu);
+  if (in) {
+    WideNode N = {};
+    N.node0 = base[0] + (before & 0xFFFFu);
+    N.tri0 = base[1] + (before >> 16);
+    uint32_t node_at = N.node0, tri_at = N.tri0;
+    float* plane = reinterpret_cast<float*>(N.plane);  // [6][4]
+    const float inf = __int_as_float(0x7F800000);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      if (s >= k) {
+        for (int a = 0; a < 3; ++a) {
+          plane[8 * a + s] = inf;
+          plane[8 * a + 4 + s] = -inf;
+        }
         continue;
       }
-      const uint32_t t = order[x];
-      const float4 v0 = tri[size_t(t) * 3], v1 = tri[size_t(t) * 3 + 1], v2 = tri[size_t(t) * 3 + 2];
-      float4* out = leaf + size_t(tri_at++) * 3;
-      out[0] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(t));
-      out[1] = make_float4(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z, 0.0f);
-      out[2] = make_float4(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z, 0.0f);
+      const float l3[3] = {lo[s].x, lo[s].y, lo[s].z}, h3[3] = {hi[s].x, hi[s].y, hi[s].z};
+      for (int a = 0; a < 3; ++a) {
+        const float pad = fmaxf(fabsf(l3[a]), fabsf(h3[a])) * 1e-6f;
+        plane[8 * a + s] = l3[a] > -kFarthest ? l3[a] - pad : -inf;
+        plane[8 * a + 4 + s] = h3[a] < kFarthest ? h3[a] + pad : inf;
+      }
+      const uint32_t below = __float_as_uint(lo[s].w);
+      if (below > kLeafTris) {
+        N.contents |= 1u << (24 + s);
+        cluster_of[node_at++] = c[s];
+        continue;
+      }
+      N.contents |= ((1u << below) - 1u) << (3 * s);
+      uint32_t x = c[s];  // three triangles or two are pairs over the triangles: each step takes one off
+      for (uint32_t r = below; r > 1; --r) {
+        const uint2 ch = C.child[x - C.n];
+        const bool inner = ch.x >= C.n;
+        leaf_of[tri_at++] = inner ? ch.y : ch.x;
+        x = inner ? ch.x : ch.y;
+      }
+      leaf_of[tri_at++] = x;
     }
+    wide[first + t] = N;
   }
-  wide[w] = N;
+  __syncthreads();  // the children's clusters are written, base and sums free
+  return next;
 }
 
-__global__ void __launch_bounds__(128) widen_kernel(Clusters C, uint32_t* cluster_of, int level, const uint32_t* order,
-                                                    const float4* tri, WideNode* wide, float4* leaf) {
-  const uint32_t end = C.counters[kLevelEnd + level + 1];
-  for (uint32_t w = C.counters[kLevelEnd + level] + blockIdx.x * 128u + threadIdx.x; w < end; w += gridDim.x * 128u)
-    widen(C, cluster_of, w, order, tri, wide, leaf);
+// The wide tree from its root, node 0, level by level in two launches: one block until
+// a level has kFrontierNodes nodes, then a block for each node of that level with
+// everything below it. (A launch a level and a read-back every four took 129 us for
+// 462 triangles and 360 for 522,254.)
+constexpr uint32_t kFrontierNodes = 512, kMaxFrontier = 4 * kFrontierNodes, kWidenThreads = 64;
+__global__ void __launch_bounds__(kFrontierNodes)
+    widen_top_kernel(Clusters C, const uint2* root, uint32_t* cluster_of, uint32_t* counters, WideNode* wide, uint32_t* leaf_of) {
+  if (threadIdx.x == 0) cluster_of[0] = root->x;
+  __syncthreads();
+  uint2 range = make_uint2(0u, 1u);
+  while (range.y > 0 && range.y < kFrontierNodes)
+    range = widen<kFrontierNodes>(C, cluster_of, counters, range.x, range.y, wide, leaf_of);
+  if (threadIdx.x == 0) {
+    counters[kFrontier] = range.x;
+    counters[kFrontier + 1] = range.y;
+  }
+}
+__global__ void __launch_bounds__(kWidenThreads)
+    widen_kernel(Clusters C, uint32_t* cluster_of, uint32_t* counters, WideNode* wide, uint32_t* leaf_of) {
+  __shared__ uint2 todo[kStack + 2];  // ranges of nodes; at most one a level
+  if (blockIdx.x >= counters[kFrontier + 1]) return;
+  int sp = 0;
+  uint2 range = make_uint2(counters[kFrontier] + blockIdx.x, 1u);
+  while (true) {
+    const uint32_t part = min(range.y, kWidenThreads);
+    const uint2 next = widen<kWidenThreads>(C, cluster_of, counters, range.x, part, wide, leaf_of);
+    if (range.y > part) {
+      if (threadIdx.x == 0) todo[sp] = make_uint2(range.x + part, range.y - part);
+      ++sp;
+      __syncthreads();
+    }
+    if (next.y > 0) {
+      range = next;
+    } else {
+      if (sp == 0) break;
+      range = todo[--sp];
+      __syncthreads();
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) leaf_kernel(uint32_t n, const uint32_t* leaf_of, const uint32_t* order, const float4* tri,
+                                                   float4* leaf) {
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t t = order[leaf_of[i]];
+  const float4 v0 = tri[size_t(t) * 3], v1 = tri[size_t(t) * 3 + 1], v2 = tri[size_t(t) * 3 + 2];
+  float4* out = leaf + size_t(i) * 3;
+  out[0] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(t));
+  out[1] = make_float4(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z, 0.0f);
+  out[2] = make_float4(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z, 0.0f);
 }
 
 float srgb_to_linear(int i) {
@@ -1279,83 +1327,70 @@ int nrc_bvh_build(const nrc_scene* scene, const nrc_instance_range* d_ranges, nr
     size_t tmp_bytes = 0, at = 0;
     uint32_t* const none = nullptr;
     e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, none, none, none, none, static_cast<int>(n));
-    const size_t kept_blocks = nn / kClusterThreads + 1;
     auto carve = [&](size_t bytes) {
       const size_t o = at;
       at += (bytes + 255) & ~size_t(255);
       return o;
     };
-    const size_t o_lo = carve(2 * nn * 16), o_hi = carve(2 * nn * 16), o_child = carve(nn * 8), o_tri = carve(nn * 48),
-                 o_keys = carve(nn * 4), o_vals = carve(nn * 4), o_keys2 = carve(nn * 4), o_vals2 = carve(nn * 4),
-                 o_nn = carve(nn * 4), o_kept = carve((kept_blocks + nn / (kClusterThreads * kClusterThreads) + 1) * 4),
-                 o_first = carve((ni + 1) * 4), o_box = carve(64), o_count = carve(kCounters * 4),
+    const size_t chunks = (nn + kChunk - 1) / kChunk;
+    const size_t o_hi = carve(2 * nn * 16), o_tri = carve(nn * 48), o_keys = carve(nn * 4), o_vals = carve(nn * 4),
+                 o_keys2 = carve(nn * 4), o_vals2 = carve(nn * 4), o_kept = carve(chunks * kKeep * 8),
+                 o_kept2 = carve((chunks + kFan - 1) / kFan * kKeep * 8), o_count = carve(chunks * 4),
+                 o_count2 = carve(chunks * 4), o_words = carve((kCounters + ni + 1) * 4),
                  o_tmp = carve(tmp_bytes ? tmp_bytes : 16);
     uint8_t* m = nullptr;
     if (e == cudaSuccess) e = cudaMalloc(&m, at);
     auto u32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(m + o); };
-    uint32_t *keys = u32(o_keys), *vals = u32(o_vals), *keys2 = u32(o_keys2), *vals2 = u32(o_vals2), *d_first = u32(o_first),
-             *box = u32(o_box);
+    uint32_t *keys = u32(o_keys), *vals = u32(o_vals), *keys2 = u32(o_keys2), *vals2 = u32(o_vals2), *counters = u32(o_words);
     float4* tri = reinterpret_cast<float4*>(m + o_tri);
-    float* cent = reinterpret_cast<float*>(m + o_lo + nn * 16);  // until the first merge writes its box there
-    if (e == cudaSuccess) e = cudaMemcpy(d_first, first.data(), (ni + 1) * 4, cudaMemcpyHostToDevice);
-    const uint32_t box_init[9] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u};  // centroid bounds; bad flag
-    const uint32_t count_init[kLevelEnd + 2] = {n, n, 0u, 1u, 0u, 0u, 0u, 1u};
-    if (e == cudaSuccess) e = cudaMemcpy(box, box_init, sizeof(box_init), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(m + o_count, count_init, sizeof(count_init), cudaMemcpyHostToDevice);
-    BuildArgs A{*scene, d_ranges, d_first, ni, n};
+    // The leaf array, written last, holds the clusters' low corners and children until
+    // then, and their upper half the centroids until the first merge.
+    float4* lo = leaf;
+    uint2* child = reinterpret_cast<uint2*>(leaf + 2 * nn);
+    float* cent = reinterpret_cast<float*>(leaf + nn);
+    // the counters, then each instance's first triangle
+    std::vector<uint32_t> words = {0u, 1u, 0u, 0u, 0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
+    words.insert(words.end(), first.begin(), first.end());
+    if (e == cudaSuccess) e = cudaMemcpy(counters, words.data(), words.size() * 4, cudaMemcpyHostToDevice);
+    BuildArgs A{*scene, d_ranges, counters + kCounters, ni, n};
     const uint32_t blocks = (n + 255) / 256;
     if (e == cudaSuccess) {
-      tri_kernel<<<blocks, 256>>>(A, tri, id, cent, box + 8);
-      bounds_kernel<<<blocks < 1024 ? blocks : 1024, 256>>>(cent, n, box);
-      morton_kernel<<<blocks, 256>>>(cent, n, box, keys, vals);
+      tri_kernel<<<blocks, 256>>>(A, tri, id, cent, counters + kBad);
+      bounds_kernel<<<blocks < 1024 ? blocks : 1024, 256>>>(cent, n, counters + kBox);
+      morton_kernel<<<blocks, 256>>>(cent, n, counters + kBox, keys, vals);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess)
       e = cub::DeviceRadixSort::SortPairs(m + o_tmp, tmp_bytes, keys, keys2, vals, vals2, static_cast<int>(n), 0, 30);
-    // the clustering, from the triangles in Morton order (vals2) to one cluster
-    Clusters C{reinterpret_cast<float4*>(m + o_lo), reinterpret_cast<float4*>(m + o_hi),
-               reinterpret_cast<uint2*>(m + o_child), u32(o_nn), u32(o_kept), static_cast<uint32_t>(kept_blocks),
-               u32(o_count), n};
-    uint32_t *ids = keys, *next = vals;
-    if (e == cudaSuccess) cluster_init_kernel<<<blocks, 256>>>(C, vals2, tri, guard, ids);
-    // (batches of passes and levels: each read-back of a count costs as much as a pass)
-    bool by_place = false;
-    for (uint32_t count = n; count > kFinishThreads && e == cudaSuccess;) {
-      const uint32_t g = (count + kClusterThreads - 1) / kClusterThreads, before = count;
-      for (int pass = 0; pass < kBatch; ++pass) {
-        nearest_kernel<<<g, kClusterThreads>>>(C, ids, pass & 1, by_place && pass == 0);
-        kept_kernel<<<g, kClusterThreads>>>(C, pass & 1);
-        merge_kernel<<<g, kClusterThreads>>>(C, ids, next, pass & 1);
-        std::swap(ids, next);
+    constexpr int kClusterSmem = kChunk * (2 * sizeof(float4) + kSearch * sizeof(float));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem);
+    if (e == cudaSuccess) {
+      // the clustering, from the triangles in Morton order (vals2) to one cluster
+      const Clusters C{lo, reinterpret_cast<float4*>(m + o_hi), child, n};
+      const uint2* in = nullptr;
+      const uint32_t* in_count = nullptr;
+      uint2 *kept = reinterpret_cast<uint2*>(m + o_kept), *kept2 = reinterpret_cast<uint2*>(m + o_kept2);
+      uint32_t *count = u32(o_count), *count2 = u32(o_count2);
+      for (uint32_t of = 0, grid = static_cast<uint32_t>(chunks); of != 1; of = grid, grid = (grid + kFan - 1) / kFan) {
+        cluster_kernel<<<grid, kChunk, kClusterSmem>>>(C, vals2, tri, guard, in, in_count, of, grid == 1 ? 1u : kKeep, kept,
+                                         grid == 1 ? counters + kLeft : count);
+        in = kept;
+        in_count = count;
+        std::swap(kept, kept2);
+        std::swap(count, count2);
       }
-      if ((e = cudaGetLastError()) == cudaSuccess)
-        e = cudaMemcpy(&count, C.counters + kCount, 4, cudaMemcpyDeviceToHost);
-      if (e == cudaSuccess && (count == 0 || count >= before)) e = cudaErrorUnknown;  // every pass merges a pair
-      by_place = count > before / 2;
+      // the wide tree; node 0 is over the last cluster
+      widen_top_kernel<<<1, kFrontierNodes>>>(C, in, keys2, counters, wide, keys);
+      widen_kernel<<<kMaxFrontier, kWidenThreads>>>(C, keys2, counters, wide, keys);
+      leaf_kernel<<<blocks, 256>>>(n, keys, vals2, tri, leaf);
+      e = cudaGetLastError();
     }
-    uint32_t* cluster_of = keys2;
-    if (e == cudaSuccess) finish_kernel<<<1, kFinishThreads>>>(C, ids, cluster_of);
-    // the wide tree, one launch per level; node 0 is over the last cluster
-    int levels = 0;
-    bool done = false;
-    while (!done && e == cudaSuccess && levels <= kStack) {
-      for (int l = 0; l < 4 && levels <= kStack; ++l, ++levels) {
-        widen_kernel<<<1216, 128>>>(C, cluster_of, levels, vals2, tri, wide, leaf);
-        e = cudaMemcpyAsync(C.counters + kLevelEnd + levels + 2, C.counters + kWide, 4, cudaMemcpyDeviceToDevice);
-      }
-      if (e == cudaSuccess) e = cudaGetLastError();
-      uint32_t ends[2];
-      if (e == cudaSuccess)
-        e = cudaMemcpy(ends, C.counters + kLevelEnd + levels, 8, cudaMemcpyDeviceToHost);
-      if (e == cudaSuccess) done = ends[0] == ends[1];
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    uint32_t bad = 0, left = 1;
-    if (e == cudaSuccess) e = cudaMemcpy(&bad, box + 8, 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(&left, C.counters + kCount, 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && !bad && (left != 1 || !done)) e = cudaErrorUnknown;  // not for any scene: see kStack
+    uint32_t done[kLeft + 1] = {0u, 0u, 0u, 0u};
+    if (e == cudaSuccess) e = cudaMemcpy(done, counters, sizeof(done), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && !done[kBad] && (done[kLeft] != 1 || done[kLeafs] != n)) e = cudaErrorUnknown;  // not for any scene
     cudaFree(m);
-    if (e == cudaSuccess && bad) {
+    if (e == cudaSuccess && done[kBad]) {
       cudaFree(B->block);
       delete B;
       return NRC_ERROR_INVALID_ARGUMENT;  // an index past the scene's buffers
