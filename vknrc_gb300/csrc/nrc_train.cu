@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(kApplyThreads) apply_kernel(const __grid_const
                                __uint_as_float(w1.z)};
   const uint32_t launch = w0.x, n = min(min(*A.d_count, A.batch_cap), A.capacity);
   const bool apply = n > 0 && w0.y != launch;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kApplyThreads - 1) {  // a thread past the last parameter
     A.words->launches = launch;
     if (apply) *A.state = st;
   }
