@@ -329,11 +329,12 @@ NRC_API int nrc_loss_gradient(const float* d_pred, const float* d_target, const 
  * Every call uses the same scratch: calls that may overlap on the GPU (other
  * streams, no ordering) race; order them. d_error (may be NULL) receives the
  * device-timeout flag; when NULL a word in the scratch is used, cleared on each
- * call, which the caller cannot read: a step that hit a bounded-wait timeout
- * changes neither parameters nor state but still returns NRC_OK, so pass d_error
- * to observe timeouts. Pointers that
- * are not aligned to their types (16 bytes for weights, entries and records;
- * 4 for the state, count and error words) return NRC_ERROR_MISALIGNED. */
+ * call, which the caller cannot read: a step whose gradient pass hit a
+ * bounded-wait timeout changes neither parameters nor state but still returns
+ * NRC_OK, so pass d_error to observe timeouts. The word is only written, never
+ * read. Pointers that are not aligned to their types (16 bytes for weights,
+ * entries and records; 4 for the state, count and error words) return
+ * NRC_ERROR_MISALIGNED. */
 NRC_API int nrc_train_noalloc(uint16_t* d_weights, uint16_t* d_use_weights, nrc_optimizer_entry* d_entries,
                               nrc_optimizer_state* d_state, const nrc_train_record* d_records, uint32_t* d_count,
                               uint32_t capacity, const nrc_config* cfg, uint32_t* d_error, void* stream);
